@@ -2,6 +2,9 @@
 #include <atomic>
 
 #include "common.cuh"
+#include <cuda.h>
+
+#include <mutex>
 
 #include <stdarg.h>
 #include <string.h>
@@ -37,6 +40,43 @@ static std::atomic<int> g_tune_gen{0};
 
 int tune_value(int knob) { return g_tune[knob].load(std::memory_order_relaxed); }
 int tune_generation() { return g_tune_gen.load(std::memory_order_relaxed); }
+
+// The current device's scratch pool, created on first use; nullptr when it cannot be.
+static cudaMemPool_t scratch_pool() {
+    constexpr int kMaxDevices = 64;
+    static std::mutex mu;
+    static cudaMemPool_t pools[kMaxDevices] = {};
+    static bool tried[kMaxDevices] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
+    std::lock_guard<std::mutex> lock(mu);
+    if (!tried[dev]) {
+        tried[dev] = true;
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool = nullptr;
+        cuuint64_t keep = kScratchKeep;
+        if (cudaMemPoolCreate(&pool, &props) == cudaSuccess) {
+            if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess)
+                pools[dev] = pool;
+            else
+                cudaMemPoolDestroy(pool);
+        }
+        if (!pools[dev]) cudaGetLastError();
+    }
+    return pools[dev];
+}
+
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t st) {
+    if (cudaMemPool_t pool = scratch_pool()) {
+        const cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, st);
+        if (e != cudaErrorMemoryAllocation) return e;
+        cudaGetLastError();  // the default pool may still hold memory that this one cannot get
+    }
+    return cudaMallocAsync(p, bytes, st);
+}
 
 }  // namespace bd
 

@@ -55,6 +55,15 @@ inline size_t plume_mask_bytes(int nx, int ny, int nz) {
     return plume_units_offset(nx, ny, nz) + plume_units_bytes(nx, ny, nz);
 }
 
+// Stream-ordered scratch of the synchronous entry points (error flags, the plume's masks and lists),
+// from one pool per device that keeps up to kScratchKeep bytes mapped between calls; what a call
+// needs beyond that goes back to the driver at the next synchronisation. The default pool keeps
+// nothing: every one of these calls ends in a synchronisation, so each call mapped and unmapped its
+// few bytes again (thermal 64x64x128, 20 substeps: 750-1520 us a call for 295 us of kernels; see
+// scratch_alloc). Safe from any thread and stream: the pool orders reuse by stream.
+constexpr unsigned long long kScratchKeep = 32ull << 20;
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t st);
+
 // Launch-shape knobs (BD_TUNE_*) and the generation counter bumped by every change.
 int tune_value(int knob);
 int tune_generation();

@@ -764,7 +764,7 @@ int pack_weights_launch(int taps, int cin, int cout, int n_off, int n_slice, int
 template <class F>
 static int run_checked(cudaStream_t st, const char* what, F launch) {
     int* err = nullptr;
-    BD_CUDA(cudaMallocAsync((void**)&err, sizeof(int), st));
+    BD_CUDA(scratch_alloc((void**)&err, sizeof(int), st));
     int host_err = 0;
     cudaError_t e = cudaMemsetAsync(err, 0, sizeof(int), st);
     int rc = e == cudaSuccess ? launch(err) : BD_OK;

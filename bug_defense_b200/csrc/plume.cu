@@ -945,7 +945,7 @@ extern "C" int bd_plume_advance(const BdPlumeParams* p, float* Ca, float* Cb, in
     }
     cudaStream_t st = as_stream(stream);
     unsigned char* scratch = nullptr;  // plume neighbourhood bytes, z lists and unit lists
-    BD_CUDA(cudaMallocAsync((void**)&scratch, plume_mask_bytes(p->nx, p->ny, p->nz), st));
+    BD_CUDA(scratch_alloc((void**)&scratch, plume_mask_bytes(p->nx, p->ny, p->nz), st));
     const int rc = plume_launch(p, Ca, Cb, n_substeps, F, in_b, st, nullptr, 1, scratch);
     cudaError_t e2 = cudaFreeAsync(scratch, st);
     cudaError_t e = cudaStreamSynchronize(st);

@@ -365,7 +365,7 @@ static void launch_substeps(const Geo& g, const AblConst& c, float* Ta, float* T
 template <typename F>
 static int with_error_flag(cudaStream_t st, const char* what, F launch) {
     int* err = nullptr;
-    BD_CUDA(cudaMallocAsync((void**)&err, sizeof(int), st));
+    BD_CUDA(scratch_alloc((void**)&err, sizeof(int), st));
     int rc = BD_OK;
     int host_err = 0;
     cudaError_t e = cudaMemsetAsync(err, 0, sizeof(int), st);
