@@ -405,7 +405,7 @@ def ours_main(args):
     from bug_defense_b200 import _lib
     kv = ctypes.c_int(0)
     _lib.call("bd_tune_get", _lib.TUNE_PLUME_KERNEL, ctypes.byref(kv))
-    plume_kernel = {4: "k_plume_direct_z", 6: "k_plume_direct_c"}.get(kv.value, "k_plume_step")
+    plume_kernel = {4: "k_plume_chain", 6: "k_plume_direct_c"}.get(kv.value, "k_plume_step")
     traffic = None
     tf = ROOT / "profiles" / "traffic.json"
     if tf.exists():

@@ -177,7 +177,7 @@ def autotune(inst, epochs_per_trial: int = 6, candidates=None, device=None, log=
     MC CTAs per SM (photons per thread) are timed by whole laser-on epochs; x-planes per CTA of the
     fused substep kernel by whole epochs with the laser off (the void domain does not change between
     trials): the plume stage runs beside MC and the substeps, so a shape that slows its own stage
-    but leaves the plume more room can win. The plume kernel and the direct kernel's x-planes per CTA are searched
+    but leaves the plume more room can win. The plume kernel and BD_TUNE_PLUME_XC are searched
     together, also by laser-off epochs; the compact kernel chooses its x-planes per stage on the
     device. Sets
     the winning values process-wide (bd_tune_set) and returns the choices with every trial's time
@@ -219,7 +219,7 @@ def autotune(inst, epochs_per_trial: int = 6, candidates=None, device=None, log=
     # the MC trials, whose laser epochs deepen the crater, come last
     single(_lib.TUNE_STENCIL_XC, False)
     single(_lib.TUNE_STENCIL_CAP, False)
-    # plume kernel x x-planes per CTA (only the one-launch-per-step grid kernel takes the knob); the
+    # plume kernel x x-planes per CTA (the knob shapes the batched stage only; the pair is searched so that a batched run is tuned too); the
     # candidates differ by a few per cent, so each is timed twice (forward, then reversed order) and
     # keeps its better time
     combos = [(int(kern), xc) for kern in cand[_lib.TUNE_PLUME_KERNEL]

@@ -27,7 +27,7 @@ inline int plume_mask_pitch(int nz) { return (nz + 15) / 16 * 16; }
 inline size_t plume_mask_only_bytes(int nx, int ny, int nz) {
     return ((size_t)nx * ny * plume_mask_pitch(nz) + 255) / 256 * 256;
 }
-// Then the live z groups of the direct plume kernel's columns (x chunk, 16-row y tile): one count
+// Then the live z groups of the columns (x chunk, 16-row y tile) of the one-step kernels: one count
 // byte per column, then per column the ascending ids of its 4-voxel z groups that hold void
 // (at most (nz + 3) / 4 <= 255 ids; sized for one x plane per chunk).
 constexpr int kPlumeZRows = 16;
@@ -36,7 +36,7 @@ inline size_t plume_zlist_bytes(int nx, int ny, int nz) {
     const size_t cols = (size_t)nx * ((ny + kPlumeZRows - 1) / kPlumeZRows);
     return (cols * (1 + (size_t)(nz + 3) / 4) + 255) / 256 * 256;
 }
-// Then the compact-order state of the direct plume kernel: 16 header words (unit count, chosen
+// Then the compact kernel's state: 16 header words (unit count, chosen
 // x planes per unit, unit count per candidate), the live-group bitmaps of every (x plane, y tile)
 // (8 words each), then the units (16 bytes: column << 5 | band and the band's 8 group ids), at
 // most one per band of every column.
@@ -51,8 +51,27 @@ inline size_t plume_units_bytes(int nx, int ny, int nz) {
     const size_t cols = (size_t)nx * ((ny + kPlumeZRows - 1) / kPlumeZRows);
     return ((16 + cols * 8) * sizeof(unsigned) + plume_unit_capacity(nx, ny, nz) * 16 + 255) / 256 * 256;
 }
-inline size_t plume_mask_bytes(int nx, int ny, int nz) {
+// Then the chained plume kernel's plan: a header, the first unit of every 16-row y tile, the
+// live-group bitmaps of every (x plane, y tile with its halo rows) (8 words each), the units (at most
+// one per started window of 30 z groups of a tile) and every unit's progress in up to kChainBlocks
+// blocks of steps.
+constexpr int kChainRows = 16;       // rows a unit writes
+constexpr int kChainBlocks = 256;    // blocks of steps per launch
+constexpr int kChainUnitBytes = 32;
+inline size_t chain_round(size_t b) { return (b + 255) / 256 * 256; }
+inline size_t plume_chain_offset(int nx, int ny, int nz) {
     return plume_units_offset(nx, ny, nz) + plume_units_bytes(nx, ny, nz);
+}
+inline size_t plume_chain_capacity(int ny, int nz) {
+    return (size_t)((ny + kChainRows - 1) / kChainRows) * (((size_t)(nz + 3) / 4) / 30 + 1);
+}
+inline size_t plume_chain_bytes(int nx, int ny, int nz) {
+    const size_t n_yt = (ny + kChainRows - 1) / kChainRows, cap = plume_chain_capacity(ny, nz);
+    return 256 + chain_round((n_yt + 1) * 4) + chain_round((size_t)nx * n_yt * 32) +
+           chain_round(cap * kChainUnitBytes) + chain_round(cap * kChainBlocks * 4);
+}
+inline size_t plume_mask_bytes(int nx, int ny, int nz) {
+    return plume_chain_offset(nx, ny, nz) + plume_chain_bytes(nx, ny, nz);
 }
 
 // Stream-ordered scratch of the synchronous entry points (error flags, the plume's masks and lists),

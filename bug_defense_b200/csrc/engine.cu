@@ -301,7 +301,7 @@ extern "C" int bd_engine_step_epoch(BdEngine* e, float power, int options, void*
         return run_stage(e, e->g_plume, &d.plume, sizeof(d.plume), graphs, on, [&](cudaStream_t s) -> int {
             int in_b = 0;
             int r = plume_launch(&d.plume, d.phase.plume, d.plume_alt, d.n_substeps, d.phase.flags, &in_b, s,
-                                 &e->dyn->void_zlimit, 0, e->plume_mask);
+                                 &e->dyn->void_zlimit, 0, e->plume_mask, &e->dyn->err);
             if (r) return r;
             if (in_b)
                 BD_CUDA(cudaMemcpyAsync(d.phase.plume, d.plume_alt, sizeof(float) * nv, cudaMemcpyDeviceToDevice, s));

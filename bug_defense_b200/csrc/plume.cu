@@ -3,19 +3,20 @@
 // centre), Dirichlet 0 on the outer walls, clamped at 0, optional first-order decay.
 //
 // Kernels (all evaluate the same per-voxel expression, ftcs1 / ftcs4, so they are bit-identical):
-//   k_plume_direct_z  default (BD_PLUME_KERNEL_DIRECT): one launch per step, a CTA per 32 (z) x 16 (y)
-//                     tile column marching x planes over the column's live z groups
-//   k_plume_direct_c  (BD_PLUME_KERNEL_COMPACT): the same per-unit code, one wave of CTAs looping
-//                     over a compact list of the live units, x planes per unit chosen per stage
-//   k_plume_step      any grid (nz % 4 != 0): one voxel per thread
+//   k_plume_chain     default (BD_PLUME_KERNEL_DIRECT): a whole stage in one launch, 4 FTCS steps per
+//                     pass over the field
+//   k_plume_direct_c  (BD_PLUME_KERNEL_COMPACT): one launch per step, one wave of CTAs looping over a
+//                     compact list of the live units, x planes per unit chosen per stage
+//   k_plume_step      grids of more than 255 z groups (nz > 1020): one voxel per thread
 // Layout: C-order (nx, ny, nz), z fastest; the neighbourhood of every voxel is one mask byte.
 #include "common.cuh"
 #include "engine.cuh"
 
 #include <algorithm>
 #include <atomic>
-#include <vector>
 #include <cmath>
+#include <type_traits>
+#include <vector>
 
 namespace bd {
 
@@ -202,18 +203,17 @@ __global__ void __launch_bounds__(PM_TZ * PM_TY) k_plume_step(int nx, int ny, in
     }
 }
 
-// ---- k_plume_direct / k_plume_direct_z: one launch per step --------------------------------
-// A CTA is one 32 (z) x 16 (y) tile and marches xc x planes; thread = 4 consecutive z voxels of
+// ---- one step per launch: the units of the compact and the batched kernel ---------------------
+// A unit is 16 rows (y) by 8 live z groups and marches xc x planes; thread = 4 consecutive z voxels of
 // one row, a warp 8 such groups x 4 rows (one 128-byte line per row and load). The thread keeps the
 // x-1 / x float4 of its row in registers and loads, per plane, the next plane's float4 and the
 // centre plane's y neighbours from the (L2-resident) field beside the plane's mask bytes (one
 // 32-bit load): one L2 round trip per plane, at the price of loads a tissue plane does not need. The
-// z neighbours come from the neighbouring lanes by shuffle (the tile's edge lanes load them).
-// Latency is hidden by the many independent CTAs of a step. Only void voxels are written. Needs
+// z neighbours come from the neighbouring lanes by shuffle (the unit's edge lanes load them).
+// Latency is hidden by the many independent units of a step. Only void voxels are written. Needs
 // nz % 4 == 0 and 16-byte aligned fields.
-constexpr int PL_BZ = 32;
-constexpr int PD_BY = 16;  // rows per CTA (8 * PD_BY threads)
-static_assert(PD_BY == kPlumeZRows, "z-list columns follow the direct kernel's y tiles");
+constexpr int PD_BY = 16;  // rows of a unit (8 * PD_BY threads)
+static_assert(PD_BY == kPlumeZRows, "z-list columns follow the units' y tiles");
 
 __device__ __forceinline__ void store_void(float* dst, float4 v, unsigned vd) {
     if (vd == 0x40404040u) {
@@ -226,52 +226,7 @@ __device__ __forceinline__ void store_void(float* dst, float4 v, unsigned vd) {
     }
 }
 
-__global__ void __launch_bounds__(8 * PD_BY) k_plume_direct(const float* __restrict__ C, float* __restrict__ Cn,
-                                                            const uint8_t* __restrict__ M, int nx, int ny, int nz,
-                                                            int mz, int xc, const __grid_constant__ PlumeTab k,
-                                                            const int* __restrict__ zlimit) {
-    __shared__ float w0s[64];
-    if (threadIdx.x < 64) w0s[threadIdx.x] = k.w0eff[threadIdx.x];
-    __syncthreads();
-    const int zl = zlimit ? min(max(*zlimit, 0), nz) : nz;
-    const int k0 = blockIdx.x * PL_BZ;
-    const int ib = blockIdx.z * xc, ie = min(nx, ib + xc);
-    if (k0 >= zl || ib >= ie) return;  // uniform over the CTA
-    const int zg = threadIdx.x & 7;
-    const int j = blockIdx.y * PD_BY + (threadIdx.x >> 3), z = k0 + 4 * zg;
-    const bool act = zl - z > 0 && j < ny;
-    const bool in = j < ny && z < nz;
-    const unsigned zkeep = zkeep_mask(zl, z);
-    const size_t plane = (size_t)ny * nz;
-    const size_t mplane = (size_t)ny * mz;
-    const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    size_t idx = ((size_t)ib * ny + j) * nz + z;
-    const uint8_t* mp = M + ((size_t)ib * ny + j) * mz + z;
-    float4 cw = in && ib > 0 ? __ldg(reinterpret_cast<const float4*>(C + idx - plane)) : z4;
-    float4 cc = in ? __ldg(reinterpret_cast<const float4*>(C + idx)) : z4;
-    for (int i = ib; i < ie; ++i, idx += plane, mp += mplane) {
-        const unsigned mr = act ? (__ldg(reinterpret_cast<const unsigned*>(mp)) & zkeep) : 0u;
-        const float4 ce = in && i + 1 < nx ? __ldg(reinterpret_cast<const float4*>(C + idx + plane)) : z4;
-        const float4 cs = in && j > 0 ? __ldg(reinterpret_cast<const float4*>(C + idx - nz)) : z4;
-        const float4 cn = in && j + 1 < ny ? __ldg(reinterpret_cast<const float4*>(C + idx + nz)) : z4;
-        float eb = 0.0f, et = 0.0f;
-        if (zg == 0 && in && z > 0) eb = __ldg(C + idx - 1);
-        if (zg == 7 && in && z + 4 < nz) et = __ldg(C + idx + 4);
-        const unsigned vd = mr & 0x40404040u;
-        if (__any_sync(0xffffffffu, act && vd)) {
-            float zb = __shfl_up_sync(0xffffffffu, cc.w, 1, 8);
-            float zt = __shfl_down_sync(0xffffffffu, cc.x, 1, 8);
-            if (zg == 0) zb = eb;
-            if (zg == 7) zt = et;
-            const float4 v = ftcs4(cc, cw, ce, cs, cn, zb, zt, mr, k, w0s);
-            if (act && vd) store_void(Cn + idx, v, vd);
-        }
-        cw = cc;
-        cc = ce;
-    }
-}
-
-// Live z groups of every (x chunk, y tile) column of the direct kernel: a CTA per column (grid
+// Live z groups of every (x chunk, y tile) column of units: a CTA per column (grid
 // n_yt x n_chunks), thread g = the 4-voxel z group g; live when any of the column's planes and rows
 // holds a void voxel in the group below the void z-limit (the mask bytes at or above it are not
 // rebuilt, so they are masked off here). The void domain is fixed within a plume stage, so the
@@ -313,7 +268,7 @@ __global__ void __launch_bounds__(256) k_plume_zlist(const uint8_t* __restrict__
     }
 }
 
-// One unit of the direct kernel: band `band` of column `col` (y tile yt, x chunk xch of xc planes)
+// One unit: band `band` of column `col` (y tile yt, x chunk xch of xc planes)
 // takes the column's live groups 8 band .. 8 band + 7 from its z list instead of 8 consecutive
 // groups, so z tiles that are partly tissue cost only their void groups. A lane whose z neighbour
 // group is not held by the neighbouring lane loads that neighbour voxel instead of taking it by
@@ -380,23 +335,7 @@ __device__ __forceinline__ void plume_direct_unit(const float* __restrict__ C, f
     plume_unit_groups(C, Cn, M, nx, ny, nz, mz, xc, k, zl, g, yt, xch, w0s);
 }
 
-// BD_PLUME_KERNEL_DIRECT: grid (bands, y tiles, x chunks); CTAs past a column's live bands exit at once.
-__global__ void __launch_bounds__(8 * PD_BY, 9) k_plume_direct_z(const float* __restrict__ C, float* __restrict__ Cn,
-                                                                 const uint8_t* __restrict__ M, int nx, int ny,
-                                                                 int nz, int mz, int xc,
-                                                                 const __grid_constant__ PlumeTab k,
-                                                                 const int* __restrict__ zlimit,
-                                                                 const uint8_t* __restrict__ zlist) {
-    __shared__ float w0s[64];
-    if (threadIdx.x < 64) w0s[threadIdx.x] = k.w0eff[threadIdx.x];
-    __syncthreads();
-    const int zl = zlimit ? min(max(*zlimit, 0), nz) : nz;
-    const int col = blockIdx.z * gridDim.y + blockIdx.y;
-    plume_direct_unit(C, Cn, M, nx, ny, nz, mz, xc, k, zl, zlist, gridDim.y * gridDim.z, col, blockIdx.y, blockIdx.z,
-                      blockIdx.x, w0s);
-}
-
-// ---- BD_PLUME_KERNEL_COMPACT: the direct kernel over a compact list of live units ------------
+// ---- BD_PLUME_KERNEL_COMPACT: a compact list of live units, one launch per step --------------
 // A step's CTAs are dispatched at a limited rate and the step ends with its last CTA, so the step is
 // fastest when the live units about fill one wave of resident CTAs: each CTA then runs exactly one
 // unit, and no empty CTA is dispatched between working ones. Once per stage the x planes per unit
@@ -587,6 +526,487 @@ __global__ void __launch_bounds__(8 * PD_BY * kPlumeUnitsPerCta, 3) k_plume_dire
     }
 }
 
+// ---- BD_PLUME_KERNEL_DIRECT: a chain of blocks of S FTCS steps in one launch -------------------
+// One step moves 9 bytes per void voxel for 13 operations; a launch per step spends its time on
+// dispatch and L2 round trips, and a launch per few steps recomputes the halo planes of every x
+// chunk. Here a stage is one launch. A unit is 16 rows (y) by up to 32 consecutive 4-voxel groups
+// (z) over the x range where they hold void. A CTA advances a unit by S steps while it marches once
+// along x with the time levels staggered by one plane: when plane p arrives, level 1 is computed on
+// plane p-1, level 2 on p-2, ... and level S is written for plane p-S. The next S steps of the same
+// unit are another CTA's, which follows a few planes behind: it reads what the units of its own and
+// the two neighbouring row tiles have written, as far as their progress counters say. Only the row
+// halo (4 on each side) is computed twice; nothing is recomputed along x.
+//
+// A CTA takes (block of steps, unit) pairs by a ticket, blocks in order, and waits only on the block
+// before its own, that is on lower tickets, whose CTAs are running or done: the lowest unfinished
+// ticket never waits, whatever else occupies the GPU. Every wait is bounded and raises *err.
+// Two buffers do: a unit writes plane q of block j over block j - 2's after its inputs up to plane
+// q + S are there, and the units of block j - 1 that read plane q have by then written plane q + S.
+//
+// A warp holds two rows (lane = z group); the planes a level needs stay in registers, z neighbours
+// come by shuffle, and the rows above and below a warp's pair come from shared memory, where every
+// level's plane was put one iteration earlier: one barrier per plane for all S levels. Each voxel is
+// evaluated by the same expression as everywhere else (ftcs4), so the bits depend neither on S nor
+// on the tiling; what the row halo recomputes is discarded. Groups outside a unit's are solid, or
+// its first and last are halo groups: a run of live groups longer than 32 is split into windows
+// that overlap by one group on each side (S <= 4 voxels).
+//
+// What bounds it: 12 warps of 168 registers fill an SM, and their FMA, shared-memory and issue slots
+// are each about half busy (issue 47 %, 417 instructions per warp and plane); DRAM 1 %, L2 13 %.
+// Measured on 3.58 M void voxels of 200 x 200 x 192, 680 steps: 4.16 ms, against 8.45 ms for one
+// launch per step (k_plume_direct_c), 6.4 ms for one launch per 4 steps with x chunks and their halo
+// planes, and 4.4 - 5.6 ms for 2 or 3 steps per pass, 1 row per warp or 16 warps of 128 registers.
+// Laser-off epoch of the full-resolution run 9.38 -> 6.01 ms, 48 x 48 x 144 laser-on 3.08 -> 2.18 ms.
+constexpr int kChainHalo = 4;                                  // halo rows; at most as many steps per block
+constexpr int kChainR = 2;                                     // rows of a warp
+constexpr int kChainWarps = (kChainRows + 2 * kChainHalo) / kChainR;
+constexpr int kChainThreads = 32 * kChainWarps;
+constexpr int chain_smem_bytes(int S) { return 2 * S * 2 * kChainWarps * 32 * (int)sizeof(float4); }
+constexpr unsigned kChainPolls = 1u << 22;                     // polls of ~0.7 us: about 3 s, then an error
+constexpr int kChainDone = 0x7fffffff;
+
+struct ChainUnit {
+    int tile, first, lo, hi;   // y tile; first group loaded; groups written
+    int ix0, ix1, _p0, _p1;    // planes on which the written groups may hold void
+};
+static_assert(sizeof(ChainUnit) == kChainUnitBytes, "unit records fill their region");
+
+// Regions of a stage's plan in its scratch.
+struct ChainPlan {
+    unsigned* hdr;       // [0] units, [1] ticket
+    int* tile_start;     // first unit of each y tile, and the end
+    unsigned* bits;      // live groups of (x plane, y tile with its halo rows)
+    ChainUnit* units;
+    int* progress;       // [block][unit]: planes below this are written
+    int cap;
+};
+
+static ChainPlan chain_plan(uint8_t* mask, int nx, int ny, int nz) {
+    ChainPlan p;
+    const size_t n_yt = (ny + kChainRows - 1) / kChainRows;
+    uint8_t* at = mask + plume_chain_offset(nx, ny, nz);
+    p.hdr = reinterpret_cast<unsigned*>(at);
+    at += 256;
+    p.tile_start = reinterpret_cast<int*>(at);
+    at += chain_round((n_yt + 1) * sizeof(int));
+    p.bits = reinterpret_cast<unsigned*>(at);
+    at += chain_round((size_t)nx * n_yt * kPlumeBitWords * sizeof(unsigned));
+    p.units = reinterpret_cast<ChainUnit*>(at);
+    at += chain_round(plume_chain_capacity(ny, nz) * sizeof(ChainUnit));
+    p.progress = reinterpret_cast<int*>(at);
+    p.cap = (int)plume_chain_capacity(ny, nz);
+    return p;
+}
+
+__device__ __forceinline__ int ld_acquire(const int* p) {
+    int v;
+    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_release(int* p, int v) {
+    asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// Waits until *p > plane; false when the polls run out or another wait already has.
+__device__ __forceinline__ bool chain_wait(const int* p, int plane, int& seen, int* err) {
+    for (unsigned it = 0; it < kChainPolls; ++it) {
+        seen = ld_acquire(p);
+        if (seen > plane) return true;
+        if ((it & 255u) == 255u && ld_acquire(err) != 0) return false;
+    }
+    atomicExch(err, 1);
+    return false;
+}
+
+// The field is written by other SMs during the kernel: it is read past the L1.
+template <bool VEC>
+__device__ __forceinline__ float4 chain_load(const float* p, int left) {
+    if (VEC) return __ldcg(reinterpret_cast<const float4*>(p));
+    float4 v;                       // left: voxels of the row from p on
+    v.x = __ldcg(p);
+    v.y = left > 1 ? __ldcg(p + 1) : 0.0f;
+    v.z = left > 2 ? __ldcg(p + 2) : 0.0f;
+    v.w = left > 3 ? __ldcg(p + 3) : 0.0f;
+    return v;
+}
+
+template <bool VEC>
+__device__ __forceinline__ void chain_store(float* p, const float4& v, int left) {
+    if (VEC) {
+        __stcg(reinterpret_cast<float4*>(p), v);
+        return;
+    }
+    p[0] = v.x;
+    if (left > 1) p[1] = v.y;
+    if (left > 2) p[2] = v.z;
+    if (left > 3) p[3] = v.w;
+}
+
+// Per-voxel factors of a group from its four mask bytes: the effective centre weight, and the decay
+// (or 1) for a voxel that is updated, 0 for one that is not. A factor of exactly 1 leaves the bits.
+struct ChainFactors {
+    float2 wa, wc, da, dc;
+};
+__device__ __forceinline__ ChainFactors chain_factors(unsigned m, float decay, const float* w0eff) {
+    ChainFactors f;
+    f.wa = make_float2(w0eff[m & 0x3Fu], w0eff[(m >> 8) & 0x3Fu]);
+    f.wc = make_float2(w0eff[(m >> 16) & 0x3Fu], w0eff[(m >> 24) & 0x3Fu]);
+    f.da = make_float2((m & 0x00000080u) ? decay : 0.0f, (m & 0x00008000u) ? decay : 0.0f);
+    f.dc = make_float2((m & 0x00800000u) ? decay : 0.0f, (m & 0x80000000u) ? decay : 0.0f);
+    return f;
+}
+
+// ftcs4 with the factors at hand. The z terms are scalar: their operand pairs straddle the registers
+// of c, and pairing them up costs the moves that a packed operation saves.
+__device__ __forceinline__ float4 chain_ftcs4(const float4& c, const float4& w, const float4& e, const float4& s,
+                                              const float4& n, float zb, float zt, const ChainFactors& f,
+                                              const PlumeTab& k) {
+    const float2 wx = make_float2(k.wx, k.wx), wy = make_float2(k.wy, k.wy);
+    float2 a = __fmul2_rn(f.wa, make_float2(c.x, c.y));
+    float2 b = __fmul2_rn(f.wc, make_float2(c.z, c.w));
+    a = __ffma2_rn(wx, __fadd2_rn(make_float2(w.x, w.y), make_float2(e.x, e.y)), a);
+    b = __ffma2_rn(wx, __fadd2_rn(make_float2(w.z, w.w), make_float2(e.z, e.w)), b);
+    a = __ffma2_rn(wy, __fadd2_rn(make_float2(s.x, s.y), make_float2(n.x, n.y)), a);
+    b = __ffma2_rn(wy, __fadd2_rn(make_float2(s.z, s.w), make_float2(n.z, n.w)), b);
+    a.x = __fmaf_rn(k.wt, c.y, __fmaf_rn(k.wb, zb, a.x));
+    a.y = __fmaf_rn(k.wt, c.z, __fmaf_rn(k.wb, c.x, a.y));
+    b.x = __fmaf_rn(k.wt, c.w, __fmaf_rn(k.wb, c.y, b.x));
+    b.y = __fmaf_rn(k.wt, zt, __fmaf_rn(k.wb, c.z, b.y));
+    a = __fmul2_rn(a, f.da);
+    b = __fmul2_rn(b, f.dc);
+    return make_float4(fmaxf(a.x, 0.0f), fmaxf(a.y, 0.0f), fmaxf(b.x, 0.0f), fmaxf(b.y, 0.0f));
+}
+
+template <int S, bool VEC>
+__global__ void __launch_bounds__(kChainThreads, 1) k_plume_chain(float* Ca, float* Cb,
+                                                                  const uint8_t* __restrict__ M, int nx, int ny,
+                                                                  int nz, int mz, const __grid_constant__ PlumeTab k,
+                                                                  const int* __restrict__ zlimit, ChainPlan plan,
+                                                                  int nblocks, int* err) {
+    constexpr int R = kChainR;
+    extern __shared__ float4 lev[];  // [plane parity][level][warp][first, last row][lane]
+    __shared__ float w0s[64];
+    __shared__ int ticket_s;
+    constexpr int kPar = S * kChainWarps * 2 * 32;
+    if (threadIdx.x < 64) w0s[threadIdx.x] = k.w0eff[threadIdx.x];
+    const int nu = (int)__ldg(&plan.hdr[0]);
+    const int zl = zlimit ? min(max(*zlimit, 0), nz) : nz;
+    const int n_yt = (ny + kChainRows - 1) / kChainRows;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row0 = R * warp;
+    const int ws = max(warp - 1, 0) * 64 + 32, wn = min(warp + 1, kChainWarps - 1) * 64;
+    // levels whose rows of this warp some written row depends on
+    const int nlev = min(S, max(0, min(row0 + R - 1 - kChainHalo, kChainHalo + kChainRows - 1 - row0) + S));
+    const int plane = ny * nz, mplane = ny * mz;
+    const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (;;) {
+        __syncthreads();
+        if (threadIdx.x == 0) ticket_s = (int)atomicAdd(&plan.hdr[1], 1u);
+        __syncthreads();
+        const int ticket = ticket_s;
+        const int j = nu > 0 ? ticket / nu : nblocks;
+        if (j >= nblocks) break;
+        const int u = ticket - j * nu;
+        const ChainUnit rec = plan.units[u];
+        const float* C = (j & 1) ? Cb : Ca;
+        float* Cn = (j & 1) ? Ca : Cb;
+        // warp 0 waits for the units of the block before: those of this and the neighbouring y tiles
+        const int* up = plan.progress + (size_t)max(j - 1, 0) * plan.cap;
+        int* mine = plan.progress + (size_t)j * plan.cap + u;
+        const int d0 = plan.tile_start[max(rec.tile - 1, 0)], d1 = plan.tile_start[min(rec.tile + 2, n_yt)];
+        int seen = 0, vx0 = 0, vx1 = 0;  // of this lane's first unit
+        if (d0 + lane < d1) {
+            vx0 = plan.units[d0 + lane].ix0;
+            vx1 = plan.units[d0 + lane].ix1;
+        }
+        bool ok = true;
+        auto wait_plane = [&](int p) {
+            if (j == 0 || !ok) return;
+            if (p >= vx0 && p < vx1 && seen <= p) ok = chain_wait(up + d0 + lane, p, seen, err);
+            for (int v = d0 + lane + 32; v < d1; v += 32) {
+                int s2 = 0;
+                if (ok && p >= plan.units[v].ix0 && p < plan.units[v].ix1) ok = chain_wait(up + v, p, s2, err);
+            }
+            ok = __all_sync(0xffffffffu, ok);
+        };
+        const int ib = rec.ix0, ie = rec.ix1;
+        const int y0 = rec.tile * kChainRows - kChainHalo + row0;
+        const int g = rec.first + lane, z = 4 * g;
+        const unsigned keep = zkeep_mask(zl, z);
+        unsigned inr = 0u, wrr = 0u;   // bit r: row r is in the grid / written
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            if (z < nz && y0 + r >= 0 && y0 + r < ny) {
+                inr |= 1u << r;
+                if (g >= rec.lo && g <= rec.hi && row0 + r >= kChainHalo && row0 + r < kChainHalo + kChainRows)
+                    wrr |= 1u << r;
+            }
+        }
+        const int left = nz - z;
+        const int p0 = ib - S, p1 = ie + S;
+        const float* cp = C + ((long long)p0 * plane + y0 * nz + z);      // plane p0, read only inside the grid
+        const uint8_t* mp = M + ((long long)p0 * mplane + y0 * mz + z);
+        float* dst = Cn + ((long long)ib * plane + y0 * nz + z);
+        // V[l][q]: this thread's row groups of level l, plane p - l in slot (p - l - p0) mod 3
+        float4 V[S][3][R];
+        unsigned mk[S][R];  // mask words of plane p - l - 1
+        unsigned nm[R];     // of the plane in flight
+        // the factors in use and the masks they are for: computed again only where a level's mask
+        // differs from the last one in a lane of the warp, that is near the walls of a cavity
+        unsigned cm[R];
+        ChainFactors f[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+#pragma unroll
+            for (int l = 0; l < S; ++l) {
+                V[l][0][r] = V[l][1][r] = V[l][2][r] = z4;
+                mk[l][r] = 0u;
+            }
+            nm[r] = cm[r] = 0u;
+            f[r].wa = f[r].wc = f[r].da = f[r].dc = make_float2(0.f, 0.f);
+        }
+        auto fetch = [&](int p, float4 (&e)[R]) {
+            const bool in = p >= 0 && p < nx;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                e[r] = z4;
+                nm[r] = 0u;
+                if (in && (inr >> r) & 1u) {
+                    e[r] = chain_load<VEC>(cp + r * nz, left);
+                    nm[r] = __ldg(reinterpret_cast<const unsigned*>(mp + r * mz));
+                }
+            }
+            cp += plane;
+            mp += mplane;
+        };
+        auto advance = [&](auto phase, int p) {
+            constexpr int B = 3 * S + decltype(phase)::value;
+            const int age = p - p0;
+            float4* put = lev + (p & 1) * kPar + warp * 64 + lane;
+            const float4* get = lev + ((p + 1) & 1) * kPar + lane;
+            // plane p - 1 - S was stored before the last barrier; the last warp, which has few rows to
+            // compute, publishes it
+            if (threadIdx.x == kChainThreads - 32 && age > 2 * S) st_release(mine, p - S);
+            float4 o[R];
+            unsigned m[R];  // of plane p
+#pragma unroll
+            for (int r = 0; r < R; ++r) m[r] = nm[r] & keep;
+            auto each = [&](auto fn) {
+                fn(std::integral_constant<int, 0>{});
+                if constexpr (S > 1) fn(std::integral_constant<int, 1>{});
+                if constexpr (S > 2) fn(std::integral_constant<int, 2>{});
+                if constexpr (S > 3) fn(std::integral_constant<int, 3>{});
+            };
+            each([&](auto lc) {
+                constexpr int l = decltype(lc)::value;
+                const float4(&e)[R] = V[l][(B - l) % 3];
+                const float4(&c)[R] = V[l][(B - l - 1) % 3];
+                const float4(&w)[R] = V[l][(B - l - 2) % 3];
+                put[l * kChainWarps * 64] = e[0];
+                put[l * kChainWarps * 64 + 32] = e[R - 1];
+                unsigned any = 0u, df = 0u;
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    o[r] = z4;
+                    any |= mk[l][r];
+                    df |= mk[l][r] ^ cm[r];
+                }
+                if (l < nlev && age >= 2 * (l + 1) && __any_sync(0xffffffffu, any & 0x80808080u)) {
+                    const float4 s = get[l * kChainWarps * 64 + ws];
+                    const float4 n = get[l * kChainWarps * 64 + wn];
+                    if (__any_sync(0xffffffffu, df)) {
+#pragma unroll
+                        for (int r = 0; r < R; ++r) {
+                            cm[r] = mk[l][r];
+                            f[r] = chain_factors(cm[r], k.decay, w0s);
+                        }
+                    }
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        float bz = __shfl_up_sync(0xffffffffu, c[r].w, 1);
+                        float tz = __shfl_down_sync(0xffffffffu, c[r].x, 1);
+                        if (lane == 0) bz = 0.0f;    // solid (its weight is in w0eff), or a halo group
+                        if (lane == 31) tz = 0.0f;
+                        o[r] = chain_ftcs4(c[r], w[r], e[r], r == 0 ? s : c[max(r - 1, 0)],
+                                           r == R - 1 ? n : c[min(r + 1, R - 1)], bz, tz, f[r], k);
+                    }
+                }
+                if constexpr (l + 1 < S) {
+#pragma unroll
+                    for (int r = 0; r < R; ++r) V[l + 1][(B - l - 1) % 3][r] = o[r];
+                }
+                if constexpr (l == 0) {
+                    if (p + 1 < p1) fetch(p + 1, V[0][(B + 1) % 3]);
+                }
+            });
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+#pragma unroll
+                for (int l = S - 1; l > 0; --l) mk[l][r] = mk[l - 1][r];
+                mk[0][r] = m[r];
+            }
+            if (age >= 2 * S) {
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+                    if ((wrr >> r) & 1u) chain_store<VEC>(dst + r * nz, o[r], left);  // solid voxels hold 0 already
+                dst += plane;
+            }
+            if (warp == 0) wait_plane(p + 2);  // fetched by every warp in the next iteration
+            __syncthreads();
+        };
+        if (warp == 0) {
+            for (int p = p0; p < p0 + 2; ++p) wait_plane(p);
+        }
+        __syncthreads();
+        fetch(p0, V[0][0]);
+        for (int p = p0; p < p1;) {
+            advance(std::integral_constant<int, 0>{}, p);
+            if (++p >= p1) break;
+            advance(std::integral_constant<int, 1>{}, p);
+            if (++p >= p1) break;
+            advance(std::integral_constant<int, 2>{}, p);
+            ++p;
+        }
+        if (threadIdx.x == 0) st_release(mine, kChainDone);
+    }
+}
+
+// bit g of (x plane, y tile): a voxel of group g below the void z-limit is void in the tile's rows or
+// its halo rows. CTA per (y tile, x plane), a warp per row, 32 groups a pass.
+__global__ void __launch_bounds__(256) k_plume_chain_bits(const uint8_t* __restrict__ M, int ny, int nz, int mz,
+                                                          const int* __restrict__ zlimit,
+                                                          unsigned* __restrict__ bits) {
+    __shared__ unsigned w8[kPlumeBitWords];
+    const int zl = zlimit ? min(max(*zlimit, 0), nz) : nz;
+    if (threadIdx.x < kPlumeBitWords) w8[threadIdx.x] = 0u;
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int j0 = max(0, (int)blockIdx.x * kChainRows - kChainHalo);
+    const int j1 = min(ny, (int)(blockIdx.x + 1) * kChainRows + kChainHalo);
+    for (int w = 0; 128 * w < zl; ++w) {
+        const int z = 128 * w + 4 * lane;
+        unsigned m = 0u;
+        if (z < zl)
+            for (int j = j0 + warp; j < j1; j += 8)
+                m |= __ldg(reinterpret_cast<const unsigned*>(M + ((size_t)blockIdx.y * ny + j) * mz + z));
+        const unsigned bal = __ballot_sync(0xffffffffu, (m & zkeep_mask(zl, z) & 0x40404040u) != 0u);
+        if (lane == 0 && bal) atomicOr(&w8[w], bal);
+    }
+    __syncthreads();
+    if (threadIdx.x < kPlumeBitWords)
+        bits[((size_t)blockIdx.y * gridDim.x + blockIdx.x) * kPlumeBitWords + threadIdx.x] = w8[threadIdx.x];
+}
+
+__device__ __forceinline__ bool chain_bit(const unsigned* o, int g) { return (o[g >> 5] >> (g & 31)) & 1u; }
+
+// The stage's units, one CTA: a warp ORs a y tile's live groups over x, cuts them into windows of 32
+// groups and finds the x range of each.
+__global__ void __launch_bounds__(1024) k_plume_chain_units(ChainPlan plan, int nx, int n_yt, int G) {
+    __shared__ unsigned live[32][kPlumeBitWords];
+    __shared__ int count[32];
+    __shared__ int base;
+    if (threadIdx.x == 0) base = 0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int t0 = 0; t0 < n_yt; t0 += 32) {
+        const int t = t0 + warp;
+        __syncthreads();
+        if (t < n_yt) {
+            unsigned o[kPlumeBitWords] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+            for (int i = lane; i < nx; i += 32) {
+                const uint4* b = reinterpret_cast<const uint4*>(plan.bits + ((size_t)i * n_yt + t) * kPlumeBitWords);
+                const uint4 q = __ldg(b), r = __ldg(b + 1);
+                o[0] |= q.x; o[1] |= q.y; o[2] |= q.z; o[3] |= q.w;
+                o[4] |= r.x; o[5] |= r.y; o[6] |= r.z; o[7] |= r.w;
+            }
+#pragma unroll
+            for (int w = 0; w < kPlumeBitWords; ++w) {
+                const unsigned v = __reduce_or_sync(0xffffffffu, o[w]);
+                if (lane == 0) live[warp][w] = v;
+            }
+        }
+        __syncwarp();
+        // windows of this tile: counted first, then written behind those of the tiles before
+        for (int pass = 0; pass < 2; ++pass) {
+            int at = 0;
+            if (pass == 1) {
+                at = base;
+                for (int w = 0; w < warp; ++w) at += count[w];
+                if (t < n_yt && lane == 0) plan.tile_start[t] = at;
+            }
+            int n = 0;
+            for (int g = 0; t < n_yt && g < G;) {
+                const unsigned* o = live[warp];
+                if (!chain_bit(o, g)) {
+                    ++g;
+                    continue;
+                }
+                const int first = g > 0 && chain_bit(o, g - 1) ? g - 1 : g;  // a live group before: one halo group
+                int last = min(G - 1, first + 31);
+                if (last + 1 < G && last > g && chain_bit(o, last) && chain_bit(o, last + 1)) --last;  // one after
+                if (pass == 1) {
+                    int lo = nx, hi = 0;
+                    for (int i = lane; i < nx; i += 32) {
+                        bool any = false;
+                        for (int w = g >> 5; w <= (last >> 5); ++w) {
+                            unsigned v = __ldg(plan.bits + ((size_t)i * n_yt + t) * kPlumeBitWords + w);
+                            if (w == (g >> 5)) v &= 0xffffffffu << (g & 31);
+                            if (w == (last >> 5)) v &= 0xffffffffu >> (31 - (last & 31));
+                            any |= v != 0u;
+                        }
+                        if (any) {
+                            lo = min(lo, i);
+                            hi = max(hi, i + 1);
+                        }
+                    }
+                    lo = __reduce_min_sync(0xffffffffu, lo);
+                    hi = __reduce_max_sync(0xffffffffu, hi);
+                    if (lane == 0) plan.units[at + n] = ChainUnit{t, first, g, last, lo, hi, 0, 0};
+                }
+                ++n;
+                g = last + 1;
+            }
+            if (pass == 0) {
+                if (lane == 0) count[warp] = n;
+                __syncthreads();
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int w = 0; w < 32; ++w) base += count[w];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        plan.tile_start[n_yt] = base;
+        plan.hdr[0] = (unsigned)base;
+        plan.hdr[1] = 0u;
+    }
+}
+
+template <int S, bool VEC>
+static cudaError_t chain_launch(int slots, float* Ca, float* Cb, const uint8_t* mask, int nx, int ny, int nz, int mz,
+                                const PlumeTab& tab, const int* zl, const ChainPlan& plan, int nblocks, int* err,
+                                cudaStream_t st) {
+    constexpr int smem = chain_smem_bytes(S);
+    cudaError_t e = cudaFuncSetAttribute(k_plume_chain<S, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) e = cudaMemsetAsync(plan.hdr + 1, 0, sizeof(unsigned), st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(plan.progress, 0, sizeof(int) * (size_t)plan.cap * nblocks, st);
+    if (e != cudaSuccess) return e;
+    k_plume_chain<S, VEC><<<slots, kChainThreads, smem, st>>>(Ca, Cb, mask, nx, ny, nz, mz, tab, zl, plan, nblocks,
+                                                              err);
+    return cudaGetLastError();
+}
+
+template <bool VEC>
+static cudaError_t chain_blocks(int S, int slots, float* Ca, float* Cb, const uint8_t* mask, int nx, int ny, int nz,
+                                int mz, const PlumeTab& tab, const int* zl, const ChainPlan& plan, int nblocks,
+                                int* err, cudaStream_t st) {
+    switch (S) {
+        case 4: return chain_launch<4, VEC>(slots, Ca, Cb, mask, nx, ny, nz, mz, tab, zl, plan, nblocks, err, st);
+        case 3: return chain_launch<3, VEC>(slots, Ca, Cb, mask, nx, ny, nz, mz, tab, zl, plan, nblocks, err, st);
+        case 2: return chain_launch<2, VEC>(slots, Ca, Cb, mask, nx, ny, nz, mz, tab, zl, plan, nblocks, err, st);
+        default: return chain_launch<1, VEC>(slots, Ca, Cb, mask, nx, ny, nz, mz, tab, zl, plan, nblocks, err, st);
+    }
+}
+
 int plume_policy_steps(const BdPlumeParams* p, int* n_steps, float* dt_step, float* decay_step) {
     const double idx2 = 1.0 / ((double)p->dx * p->dx), idy2 = 1.0 / ((double)p->dy * p->dy);
     const double idz2 = 1.0 / ((double)p->dz * p->dz);
@@ -640,7 +1060,7 @@ static int compact_slots() {
 // non-void voxels may hold anything) the mask covers the whole grid and the non-void voxels of both
 // buffers are set to 0 first (every step keeps them 0).
 int plume_launch(const BdPlumeParams* p, float* Ca, float* Cb, int n_substeps, const uint8_t* F, int* in_b,
-                 cudaStream_t st, const int* zlimit, int full_first, uint8_t* mask) {
+                 cudaStream_t st, const int* zlimit, int full_first, uint8_t* mask, int* err) {
     int steps;
     float dtp, decay;
     int rc = plume_policy_steps(p, &steps, &dtp, &decay);
@@ -665,7 +1085,7 @@ int plume_launch(const BdPlumeParams* p, float* Ca, float* Cb, int n_substeps, c
     }
     const long long total = (long long)steps * n_substeps;
     const int kernel = tune_value(BD_TUNE_PLUME_KERNEL);
-    const bool vec = nz % 4 == 0;  // the direct kernels move float4 groups
+    const bool vec = nz % 4 == 0;  // rows of whole float4 groups
     if (kernel == BD_PLUME_KERNEL_COMPACT && vec && (nz + 3) / 4 <= 255) {
         const int n_yt = (ny + PD_BY - 1) / PD_BY;
         unsigned* hdr = reinterpret_cast<unsigned*>(mask + plume_units_offset(nx, ny, nz));
@@ -690,26 +1110,36 @@ int plume_launch(const BdPlumeParams* p, float* Ca, float* Cb, int n_substeps, c
         if (in_b) *in_b = (int)(total & 1);
         return BD_OK;
     }
-    const int xc = tune_value(BD_TUNE_PLUME_XC);
-    const dim3 dgrid((nz + PL_BZ - 1) / PL_BZ, (ny + PD_BY - 1) / PD_BY, (nx + xc - 1) / xc);
-    // live z groups per direct-kernel column, from this stage's mask
-    uint8_t* zlist = nullptr;
-    if (vec && (nz + 3) / 4 <= 255) {
-        zlist = mask + plume_zlist_offset(nx, ny, nz);
-        k_plume_zlist<<<dim3((ny + PD_BY - 1) / PD_BY, (nx + xc - 1) / xc), 256, 0, st>>>(mask, nx, ny, nz, mz, xc, zl,
-                                                                                          zlist);
-        BD_CHECK_LAUNCH("k_plume_zlist");
+    if ((nz + 3) / 4 <= 255) {
+        const int n_yt = (ny + kChainRows - 1) / kChainRows;
+        const ChainPlan plan = chain_plan(mask, nx, ny, nz);
+        int dev = 0, nsm = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+        const int slots = std::max(1, nsm);
+        k_plume_chain_bits<<<dim3(n_yt, nx), 256, 0, st>>>(mask, ny, nz, mz, zl, plan.bits);
+        k_plume_chain_units<<<1, 1024, 0, st>>>(plan, nx, n_yt, (nz + 3) / 4);
+        BD_CHECK_LAUNCH("k_plume_chain_units");
+        int flips = 0;
+        for (long long left = total; left > 0;) {
+            const int S = (int)std::min<long long>(left, kChainHalo);
+            const int nb = (int)std::min<long long>(left / S, kChainBlocks);
+            float* a = (flips & 1) ? Cb : Ca;
+            float* b = (flips & 1) ? Ca : Cb;
+            const cudaError_t e = vec ? chain_blocks<true>(S, slots, a, b, mask, nx, ny, nz, mz, tab, zl, plan, nb, err, st)
+                                      : chain_blocks<false>(S, slots, a, b, mask, nx, ny, nz, mz, tab, zl, plan, nb, err, st);
+            if (e != cudaSuccess) return cuda_status(e, "k_plume_chain");
+            flips += nb;
+            left -= (long long)S * nb;
+        }
+        if (in_b) *in_b = flips & 1;
+        return BD_OK;
     }
     for (long long s = 0; s < total; ++s) {
         const float* in = (s & 1) ? Cb : Ca;
         float* out = (s & 1) ? Ca : Cb;
-        if (zlist)
-            k_plume_direct_z<<<dgrid, 8 * PD_BY, 0, st>>>(in, out, mask, nx, ny, nz, mz, xc, tab, zl, zlist);
-        else if (vec)
-            k_plume_direct<<<dgrid, 8 * PD_BY, 0, st>>>(in, out, mask, nx, ny, nz, mz, xc, tab, zl);
-        else
-            k_plume_step<<<dim3((ny + PM_TY - 1) / PM_TY, nx), dim3(PM_TZ, PM_TY), 0, st>>>(nx, ny, nz, mz, tab, in, out,
-                                                                                        mask, zl);
+        k_plume_step<<<dim3((ny + PM_TY - 1) / PM_TY, nx), dim3(PM_TZ, PM_TY), 0, st>>>(nx, ny, nz, mz, tab, in, out, mask,
+                                                                                        zl);
     }
     BD_CHECK_LAUNCH("k_plume_step");
     if (in_b) *in_b = (int)(total & 1);
@@ -944,14 +1374,20 @@ extern "C" int bd_plume_advance(const BdPlumeParams* p, float* Ca, float* Cb, in
         return BD_OK;
     }
     cudaStream_t st = as_stream(stream);
-    unsigned char* scratch = nullptr;  // plume neighbourhood bytes, z lists and unit lists
-    BD_CUDA(scratch_alloc((void**)&scratch, plume_mask_bytes(p->nx, p->ny, p->nz), st));
-    const int rc = plume_launch(p, Ca, Cb, n_substeps, F, in_b, st, nullptr, 1, scratch);
+    unsigned char* scratch = nullptr;  // an error flag, then the plume neighbourhood bytes and plans
+    BD_CUDA(scratch_alloc((void**)&scratch, 256 + plume_mask_bytes(p->nx, p->ny, p->nz), st));
+    int* err = reinterpret_cast<int*>(scratch);
+    int host_err = 0;
+    cudaError_t e = cudaMemsetAsync(err, 0, sizeof(int), st);
+    int rc = BD_OK;
+    if (e == cudaSuccess) rc = plume_launch(p, Ca, Cb, n_substeps, F, in_b, st, nullptr, 1, scratch + 256, err);
+    if (e == cudaSuccess && rc == BD_OK) e = cudaMemcpyAsync(&host_err, err, sizeof(int), cudaMemcpyDeviceToHost, st);
     cudaError_t e2 = cudaFreeAsync(scratch, st);
-    cudaError_t e = cudaStreamSynchronize(st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (rc) return rc;
     if (e != cudaSuccess) return cuda_status(e, "bd_plume_advance");
     if (e2 != cudaSuccess) return cuda_status(e2, "bd_plume_advance: cudaFreeAsync");
+    if (host_err) return fail(BD_ERR_TIMEOUT, "bd_plume_advance: a bounded device wait timed out");
     return BD_OK;
 }
 

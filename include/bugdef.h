@@ -375,18 +375,16 @@ BD_API int bd_engine_record(BdEngine* e, const BdRecordSpec* spec, void* slot, v
 #define BD_TUNE_MC_BLOCKS_PER_SM  0  /* persistent MC grid: 128-thread CTAs per SM, 1..16 (0 = occupancy
                                         limit); photons per thread = n_photons / (grid * 128)          */
 #define BD_TUNE_STENCIL_XC        1  /* x-planes per CTA of the TMA substep kernel, 1..64 (default 8)   */
-#define BD_TUNE_PLUME_XC          2  /* direct plume kernel: x-planes per CTA, 1..64 (default 4)         */
+#define BD_TUNE_PLUME_XC          2  /* batched plume stage: x-planes per unit, 1..64 (default 4)       */
 #define BD_TUNE_PLUME_KERNEL      3  /* plume stage: BD_PLUME_KERNEL_DIRECT (default) or
                                         BD_PLUME_KERNEL_COMPACT (value 5 is not used)                   */
-#define BD_PLUME_KERNEL_DIRECT    4  /* one launch per FTCS step: a CTA per 32 (z) x 16 (y) tile column
-                                        marching x planes over the column's live z groups              */
-#define BD_PLUME_KERNEL_COMPACT   6  /* the direct kernel's per-unit code over a compact list of the live
-                                        (column, band) units, one wave of CTAs per step: once per stage
-                                        the x planes per unit are chosen on the device (2..12, the
-                                        smallest whose unit count fits one wave; BD_TUNE_PLUME_XC is not
-                                        used), so no empty CTA is dispatched and no partial second wave
-                                        runs. Same results as BD_PLUME_KERNEL_DIRECT; nz % 4 != 0 falls
-                                        back to it                                                      */
+#define BD_PLUME_KERNEL_DIRECT    4  /* one launch per stage: each CTA advances 16 rows by 4 FTCS steps in
+                                        one march along x, following the CTA with the steps before      */
+#define BD_PLUME_KERNEL_COMPACT   6  /* one launch per FTCS step: one wave of CTAs over a compact list of
+                                        the live (column, band) units; once per stage the x planes per
+                                        unit are chosen on the device (2..12, the smallest whose unit
+                                        count fits one wave). Same results as BD_PLUME_KERNEL_DIRECT;
+                                        nz % 4 != 0 falls back to it                                    */
 #define BD_TUNE_STENCIL_CAP       4  /* at most this many substep CTAs per SM (0 = no cap, default): the
                                         plume stage runs beside the substeps and keeps the rest         */
 #define BD_TUNE_COUNT             5
