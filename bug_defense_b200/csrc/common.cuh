@@ -141,32 +141,66 @@ struct Philox {
         }
         return make_uint4(x0, x1, x2, x3);
     }
+    // the same with the ten round keys at hand (kernel parameters: operands straight from the constant
+    // bank, where adding them up costs two instructions a round and the two key registers)
+    __host__ static inline void keys(uint32_t k0, uint32_t k1, uint32_t* ks) {
+        for (int r = 0; r < 10; ++r) {
+            ks[2 * r] = k0; ks[2 * r + 1] = k1;
+            k0 += W0; k1 += W1;
+        }
+    }
+    __device__ static inline uint4 gen(uint4 c, const uint32_t* ks) {
+        uint32_t x0 = c.x, x1 = c.y, x2 = c.z, x3 = c.w;
+#pragma unroll
+        for (int r = 0; r < 10; ++r) round(x0, x1, x2, x3, ks[2 * r], ks[2 * r + 1]);
+        return make_uint4(x0, x1, x2, x3);
+    }
 };
 
-// Per-photon stream: counter = (photon lo, photon hi, draw block, 0x42444d43 'BDMC').
+// Per-photon stream: counter = (photon lo, photon hi, draw block, 0x42444d43 'BDMC'); draw n is word
+// n & 3 of block n >> 2. r0..r3 always hold the block of the next draw, so a draw never waits for a
+// block, and the three draws of a scattering need one block at one place: lanes whose positions in
+// their blocks differ would otherwise each run the ten rounds at another of the three draws.
+// `ks`: the round keys of the run's seed (Philox::keys).
 struct PhotonRng {
-    uint32_t k0, k1, p_lo, p_hi, blk;
-    uint32_t r0, r1, r2, r3;
-    int left;
-    __device__ inline void init(uint64_t seed, uint64_t photon) {
-        k0 = (uint32_t)seed; k1 = (uint32_t)(seed >> 32);
-        p_lo = (uint32_t)photon; p_hi = (uint32_t)(photon >> 32);
-        blk = 0; left = 0;
+    uint32_t p_lo, p_hi;
+    uint32_t n;               // draws so far
+    uint32_t r0, r1, r2, r3;  // block n >> 2
+    __device__ inline uint4 block(uint32_t b, const uint32_t* ks) const {
+        return Philox::gen(make_uint4(p_lo, p_hi, b, 0x42444d43u), ks);
     }
-    __device__ inline uint32_t next_u32() {
-        if (left == 0) {
-            uint4 v = Philox::gen(make_uint4(p_lo, p_hi, blk++, 0x42444d43u), k0, k1);
-            r0 = v.x; r1 = v.y; r2 = v.z; r3 = v.w; left = 4;
-        }
-        uint32_t out = r0;
-        r0 = r1; r1 = r2; r2 = r3; --left;
+    __device__ inline void hold(const uint4& v) { r0 = v.x; r1 = v.y; r2 = v.z; r3 = v.w; }
+    __device__ inline void init(uint64_t photon, const uint32_t* ks) {
+        p_lo = (uint32_t)photon; p_hi = (uint32_t)(photon >> 32);
+        n = 0;
+        hold(block(0, ks));
+    }
+    __device__ inline uint32_t next_u32(const uint32_t* ks) {
+        const uint32_t lo = (n & 1u) ? r1 : r0, hi = (n & 1u) ? r3 : r2;
+        const uint32_t out = (n & 2u) ? hi : lo;
+        ++n;
+        if ((n & 3u) == 0u) hold(block(n >> 2, ks));
         return out;
     }
+    // the next three draws
+    __device__ inline void next3(uint32_t& u0, uint32_t& u1, uint32_t& u2, const uint32_t* ks) {
+        const bool odd = (n & 1u) != 0u, upper = (n & 2u) != 0u, turn = (n & 3u) != 0u;
+        uint4 x = make_uint4(0u, 0u, 0u, 0u);
+        if (turn) x = block((n >> 2) + 1u, ks);
+        const uint32_t t0 = odd ? r1 : r0, t1 = odd ? r2 : r1, t2 = odd ? r3 : r2, t3 = odd ? x.x : r3,
+                       t4 = odd ? x.y : x.x;
+        u0 = upper ? t2 : t0;
+        u1 = upper ? t3 : t1;
+        u2 = upper ? t4 : t2;
+        n += 3u;
+        if (turn) hold(x);
+    }
     // uniform in [0, 1): 24 significant bits
-    __device__ inline float uniform() { return (float)(next_u32() >> 8) * (1.0f / 16777216.0f); }
+    __device__ static inline float to_uniform(uint32_t u) { return (float)(u >> 8) * (1.0f / 16777216.0f); }
+    __device__ inline float uniform(const uint32_t* ks) { return to_uniform(next_u32(ks)); }
     // uniform in (0, 1): never 0, for logarithms
-    __device__ inline float uniform_pos() {
-        return ((float)(next_u32() >> 8) + 0.5f) * (1.0f / 16777216.0f);
+    __device__ inline float uniform_pos(const uint32_t* ks) {
+        return ((float)(next_u32(ks) >> 8) + 0.5f) * (1.0f / 16777216.0f);
     }
 };
 
