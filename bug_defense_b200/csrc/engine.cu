@@ -353,7 +353,7 @@ extern "C" int bd_engine_step_epoch(BdEngine* e, float power, int options, void*
         ap.zero_src_in_ablated = 1;
         rc = run_stage(e, laser ? e->g_sub_on : e->g_sub_off, &ap, sizeof(ap), graphs, st, [&](cudaStream_t s) -> int {
             int r = ablation_launch(&ap, d.phase.T, d.T_alt, d.n_substeps, d.phase.H_acc, d.omega, d.phase.chi,
-                                    d.phase.flags, d.A, d.phase.k, d.phase.rho_cp, s, &e->dyn->err);
+                                    d.phase.flags, d.A, d.phase.k, d.phase.rho_cp, s);
             if (r) return r;
             if (d.n_substeps & 1)
                 BD_CUDA(cudaMemcpyAsync(d.phase.T, d.T_alt, sizeof(float) * nv, cudaMemcpyDeviceToDevice, s));

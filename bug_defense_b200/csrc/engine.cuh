@@ -55,7 +55,7 @@ struct PhaseArgs {
                          // no diagnostics): after the optics change mid-run
 int phase_launch(const PhaseArgs& a, int mode, cudaStream_t st);
 int ablation_launch(const BdAblationParams* p, float* Ta, float* Tb, int n, float* H, float* Om, float* Chi,
-                    const uint8_t* F, const float* src, const float* K, const float* R, cudaStream_t st, int* err);
+                    const uint8_t* F, const float* src, const float* K, const float* R, cudaStream_t st);
 int plume_launch(const BdPlumeParams* p, float* Ca, float* Cb, int n_substeps, const uint8_t* F, int* in_b,
                  cudaStream_t st, const int* zlimit, int full_first, uint8_t* mask, int* err);
 int plume_policy_steps(const BdPlumeParams* p, int* n_steps, float* dt_step, float* decay_step);

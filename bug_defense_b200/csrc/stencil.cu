@@ -9,28 +9,54 @@
 //   (coupled_ablation.py:33-40) and first-order char kinetics (coupled_ablation.py:43-58),
 //   all pointwise on the trial temperature, so one pass per substep does everything.
 //
-// Layout: z fastest. A CTA owns a 32 (z) x 8 (y) column tile and marches along x (the
-// slowest axis), rotating the x-1 / x / x+1 values of T and k through registers, so each
-// T and k value is fetched from DRAM once per substep; y/z neighbours come from L1.
+// Layout: z fastest. A thread owns 4 consecutive z voxels (a float4) of one row and marches along x
+// (the slowest axis); the plane's groups are dealt to threads in memory order, so any nz fills the
+// warps. A face's flux is computed once: +x kept for the next plane, z faces within the thread and
+// by shuffle from the lane below, only the y faces twice (their rows come from L1). The source and the
+// enthalpy are read only where a voxel uses them.
+// What bounds it: latency and issue, with DRAM behind them (200x200x192: 217 MB a substep, 4 TB/s;
+// 575 warp instructions per 32 groups of 4). 20 substeps, char on / char and damage on: 1.85 / 2.13 ms
+// by 32 x 16 tiles staged through shared memory with every face computed twice, now 1.07 / 1.33 ms
+// (5 CTAs of 128 threads per SM; 3 of 256 1.20 / 1.51, 6 of 128 1.17 / 1.46, 10 of 64 1.09 / 1.34).
+// 150x150x138 (rows of no whole float4s) 0.86 -> 0.64 ms. Same bits.
 #include "common.cuh"
-#include "tma.cuh"
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 namespace bd {
 
-constexpr int TZ = 32, TY = 8;
 
 struct Geo {
     int nx, ny, nz, ni;
     float idx2, idy2, idz2, dz, h_eff, t_amb, dt;
 };
 
-// Harmonic face conductance 2 k_c k_n / (k_c + k_n + 1e-12). The quotient uses the fast
-// reciprocal path (<= 2 ulp): six precise IEEE divisions per voxel made the stencil
-// instruction-bound, while the parity bar on T is 1e-4 relative.
-__device__ __forceinline__ float kface(float a, float b) { return __fdividef(2.0f * a * b, a + b + 1e-12f); }
+// Harmonic face conductance 2 k_c k_n / (k_c + k_n + 1e-12) by the approximate reciprocal (<= 1 ulp): six
+// precise IEEE divisions per voxel made the stencil instruction-bound, while the parity bar on T is
+// 1e-4 relative. The operations are written out: the compiler contracts none of them, so every
+// grid and every launch shape gives the same bits.
+__device__ __forceinline__ float rcp_approx(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float2 rcp_approx2(float2 x) { return make_float2(rcp_approx(x.x), rcp_approx(x.y)); }
+// conductance x temperature step across a face; k2: 2 k_c, nt: -T_c
+__device__ __forceinline__ float face(float k2, float kc, float kn, float nt, float tn) {
+    const float kf = __fmul_rn(__fmul_rn(k2, kn), rcp_approx(__fadd_rn(__fadd_rn(kc, kn), 1e-12f)));
+    return __fmul_rn(kf, __fadd_rn(tn, nt));
+}
+__device__ __forceinline__ float2 face2(float2 k2, float2 kc, float2 kn, float2 nt, float2 tn) {
+    const float2 den = __fadd2_rn(__fadd2_rn(kc, kn), make_float2(1e-12f, 1e-12f));
+    return __fmul2_rn(__fmul2_rn(__fmul2_rn(k2, kn), rcp_approx2(den)), __fadd2_rn(tn, nt));
+}
+// A product that enters a sum rounded. Scalar: a packed multiply may be contracted with the packed add
+// that takes it, a scalar one with explicit rounding is not.
+__device__ __forceinline__ float2 scale2(float2 a, float s) { return make_float2(__fmul_rn(a.x, s), __fmul_rn(a.y, s)); }
+__device__ __forceinline__ float2 lo2(const float4& v) { return make_float2(v.x, v.y); }
+__device__ __forceinline__ float2 hi2(const float4& v) { return make_float2(v.z, v.w); }
 
 template <int BC>
 __device__ __forceinline__ float zwall_flux(float Tc, float kc, const Geo& g) {
@@ -48,229 +74,247 @@ __device__ __forceinline__ float zwall_flux(float Tc, float kc, const Geo& g) {
 struct AblConst {
     float t_abl, t_void, q_scale;
     float arr_A, arr_EaR, char_A, char_EaR;
+    float t_cold;   // below this temperature a substep's char rate is nothing in FP32 (degC)
     int zero_src_in_ablated, is_active;
 };
 
-// MODE 0: thermal only. MODE 1: fused ablation substep.
-// Each thread marches NI x-planes of one (y, z) column; T and k of plane i+2 are prefetched
-// while plane i is computed so two DRAM round trips are in flight per thread.
-template <int MODE, int BC, bool ARR, bool CHAR>
-__global__ void __launch_bounds__(TZ * TY) k_substep(Geo g, AblConst c, const float* __restrict__ T,
-                                                     float* __restrict__ Tn, const float* __restrict__ src,
-                                                     const float* __restrict__ K, const float* __restrict__ R,
-                                                     const uint8_t* __restrict__ F, float* __restrict__ H,
-                                                     float* __restrict__ Om, float* __restrict__ Chi) {
-    const int k = blockIdx.x * TZ + threadIdx.x;
-    const int j = blockIdx.y * TY + threadIdx.y;
-    if (k >= g.nz || j >= g.ny) return;
-    const int i0 = blockIdx.z * g.ni;
-    const int i1 = min(i0 + g.ni, g.nx);
-    const int plane = g.ny * g.nz;
-    const int base = j * g.nz + k;
+// MODE 0: thermal only. MODE 1: fused ablation substep. A thread owns 4 consecutive z voxels (one
+// float4) of the plane's groups, taken in memory order, and marches xc planes along x.
+constexpr int SUB_T = 128;
+constexpr int SUB_WAVE = 12;   // CTAs per SM that the choice of planes per CTA aims at, at least
 
-    int idx = i0 * plane + base;
-    float Tm = 0.0f, km = 0.0f, Tp = 0.0f, kp = 0.0f;
-    float Tc = __ldg(&T[idx]), kc = __ldg(&K[idx]);
-    if (i0 > 0) { Tm = __ldg(&T[idx - plane]); km = __ldg(&K[idx - plane]); }
-    if (i0 + 1 < g.nx) { Tp = __ldg(&T[idx + plane]); kp = __ldg(&K[idx + plane]); }
-
-    for (int i = i0; i < i1; ++i, idx += plane) {
-        // prefetch plane i+2 (the x+1 neighbour of the next iteration)
-        float Tq = 0.0f, kq = 0.0f;
-        if (i + 2 < g.nx && i + 1 < i1) { Tq = __ldg(&T[idx + 2 * plane]); kq = __ldg(&K[idx + 2 * plane]); }
-        const float rho = __ldg(&R[idx]);
-        uint8_t f = 0;
-        if (MODE == 1) f = __ldg(&F[idx]);
-        float q = 0.0f;
-        if (c.is_active) q = __ldg(&src[idx]);
-
-        const bool has_e = (i + 1 < g.nx);
-        float fw = (i > 0) ? kface(kc, km) * (Tm - Tc) * g.idx2 : 0.0f;
-        float fe = has_e ? kface(kc, kp) * (Tp - Tc) * g.idx2 : 0.0f;
-        float fs = 0.0f, fn = 0.0f, ft, fb;
-        if (j > 0)        fs = kface(kc, __ldg(&K[idx - g.nz])) * (__ldg(&T[idx - g.nz]) - Tc) * g.idy2;
-        if (j + 1 < g.ny) fn = kface(kc, __ldg(&K[idx + g.nz])) * (__ldg(&T[idx + g.nz]) - Tc) * g.idy2;
-        if (k > 0)        ft = kface(kc, __ldg(&K[idx - 1])) * (__ldg(&T[idx - 1]) - Tc) * g.idz2;
-        else              ft = zwall_flux<BC>(Tc, kc, g);
-        if (k + 1 < g.nz) fb = kface(kc, __ldg(&K[idx + 1])) * (__ldg(&T[idx + 1]) - Tc) * g.idz2;
-        else              fb = zwall_flux<BC>(Tc, kc, g);
-        const float div = fw + fe + fs + fn + ft + fb;
-
-        const float cap = fmaxf(rho, 1e-12f);
-        q *= c.q_scale;
-        if (MODE == 1 && c.zero_src_in_ablated && (f & BD_FLAG_ABLATED)) q = 0.0f;
-        float Tt = Tc + __fdividef(g.dt * (div + q), cap);
-
-        if (MODE == 1) {
-            const bool abl = (f & BD_FLAG_ABLATED) != 0;
-            const bool dry = (f & BD_FLAG_DRY) != 0;
-            if (abl) {
-                if (Tt > c.t_void) Tt = c.t_void;
-            } else if (!dry) {
-                float h = H[idx];
-                if (Tt > c.t_abl) {
-                    h += (Tt - c.t_abl) * rho;
-                    Tt = c.t_abl;
-                    H[idx] = h;
-                } else if (h > 0.0f) {
-                    float rel = fminf(h, (c.t_abl - Tt) * rho);
-                    H[idx] = h - rel;
-                    Tt = Tt + rel / rho;
-                }
-            }
-            if (ARR && !abl) Om[idx] += g.dt * c.arr_A * expf(-c.arr_EaR / (Tt + 273.15f));
-            if (CHAR && dry && !abl) {
-                float rate = c.char_A * expf(-c.char_EaR / (Tt + 273.15f));
-                float x = Chi[idx];
-                Chi[idx] = 1.0f - (1.0f - x) * expf(-rate * g.dt);
-            }
-        }
-        Tn[idx] = Tt;
-        Tm = Tc; km = kc; Tc = Tp; kc = kp; Tp = Tq; kp = kq;
+// 4 voxels from p on; `left` of them (>= 1) are in the row
+template <bool VEC>
+__device__ __forceinline__ float4 load4(const float* p, int left) {
+    if (VEC) return *reinterpret_cast<const float4*>(p);
+    return make_float4(p[0], left > 1 ? p[1] : 0.0f, left > 2 ? p[2] : 0.0f, left > 3 ? p[3] : 0.0f);
+}
+template <bool VEC>
+__device__ __forceinline__ float4 load4_ro(const float* __restrict__ p, int left) {
+    if (VEC) return __ldg(reinterpret_cast<const float4*>(p));
+    return make_float4(__ldg(p), left > 1 ? __ldg(p + 1) : 0.0f, left > 2 ? __ldg(p + 2) : 0.0f,
+                       left > 3 ? __ldg(p + 3) : 0.0f);
+}
+template <bool VEC>
+__device__ __forceinline__ void store4(float* p, const float* v, int left) {
+    if constexpr (VEC) {
+        *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (i < left) p[i] = v[i];
     }
 }
+template <bool VEC>
+__device__ __forceinline__ unsigned load_flags4(const uint8_t* __restrict__ p, int left) {
+    if (VEC) return __ldg(reinterpret_cast<const unsigned*>(p));
+    unsigned f = __ldg(p);
+    if (left > 1) f |= (unsigned)__ldg(p + 1) << 8;
+    if (left > 2) f |= (unsigned)__ldg(p + 2) << 16;
+    if (left > 3) f |= (unsigned)__ldg(p + 3) << 24;
+    return f;
+}
 
-// TMA-staged fused substep: same arithmetic as k_substep, but a CTA owns a 32 (z) x 16 (y) tile
-// and marches a chunk of x planes; T and k tiles of each plane (1-voxel y halo, 4-voxel z halo)
-// stream through a 4-stage shared-memory ring filled by the TMA engine, and the per-voxel fields of
-// the next plane (rho_cp, source, flags, H) are fetched into registers one plane ahead.
-constexpr int ST_BZ = 32, ST_BY = 16, ST_PZ = ST_BZ + 8, ST_PY = ST_BY + 2, ST_STAGES = 4;
-constexpr unsigned ST_TILE_BYTES = ST_PZ * ST_PY * sizeof(float);
-constexpr int ST_STRIDE = ((ST_PZ * ST_PY * (int)sizeof(float) + 127) / 128) * 128 / (int)sizeof(float);
-static_assert(ST_STRIDE * sizeof(float) % 128 == 0, "stage stride must keep 128-byte alignment");
-
-template <int MODE, int BC, bool ARR, bool CHAR>
-__global__ void __launch_bounds__(TZ * TY) k_substep_tma(const __grid_constant__ CUtensorMap t_map,
-                                                         const __grid_constant__ CUtensorMap k_map, Geo g,
-                                                         AblConst c, float* __restrict__ Tn,
-                                                         const float* __restrict__ src, const float* __restrict__ R,
-                                                         const uint8_t* __restrict__ F, float* __restrict__ H,
-                                                         float* __restrict__ Om, float* __restrict__ Chi,
-                                                         int xc, int* __restrict__ err) {
-    __shared__ __align__(128) float ringT[ST_STAGES][ST_STRIDE];
-    __shared__ __align__(128) float ringK[ST_STAGES][ST_STRIDE];
-    __shared__ __align__(8) unsigned long long bar[ST_STAGES];
-    const int k0 = blockIdx.x * ST_BZ;
-    const int j0 = blockIdx.y * ST_BY;
-    const int ib = blockIdx.z * xc;
-    const int ie = min(g.nx, ib + xc);
-    if (ib >= ie) return;
-    const int tid = threadIdx.y * TZ + threadIdx.x;
-    if (tid == 0) {
-        for (int q = 0; q < ST_STAGES; ++q) mbar_init(&bar[q], 1);
-        mbar_init_fence();
-    }
-    __syncthreads();
-    const int nplanes = ie - ib + 2;
-    if (tid == 0) {
-        for (int q = 0; q < ST_STAGES && q < nplanes; ++q) {
-            mbar_expect_tx(&bar[q], 2 * ST_TILE_BYTES);
-            tma_load_3d(ringT[q], &t_map, k0 - 4, j0 - 1, ib - 1 + q, &bar[q]);
-            tma_load_3d(ringK[q], &k_map, k0 - 4, j0 - 1, ib - 1 + q, &bar[q]);
-        }
-    }
+template <int MODE, int BC, bool ARR, bool CHAR, bool VEC>
+__global__ void __launch_bounds__(SUB_T, 5) k_substep(Geo g, AblConst c, const float* __restrict__ T,
+                                                             float* __restrict__ Tn, const float* __restrict__ src,
+                                                             const float* __restrict__ K, const float* __restrict__ R,
+                                                             const uint8_t* __restrict__ F, float* __restrict__ H,
+                                                             float* __restrict__ Om, float* __restrict__ Chi) {
+    __shared__ float4 work[MODE == 1 && CHAR ? SUB_T / 32 : 1][16];   // per warp: 8 groups' T, 8 groups' chi
+    const int G = (g.nz + 3) / 4;
+    const int lane = threadIdx.x & 31;
+    // threads past the plane's groups work on its last one and store nothing
+    const int q0 = blockIdx.x * SUB_T + threadIdx.x, q = min(q0, g.ny * G - 1);
+    const bool on = q0 == q;
+    const int j = q / G, gi = q - j * G;
+    const int z = 4 * gi, left = g.nz - z;
     const int plane = g.ny * g.nz;
-    const int k = k0 + threadIdx.x;
-    const int jr[2] = {j0 + (int)threadIdx.y, j0 + (int)threadIdx.y + TY};
-    const bool rowok[2] = {k < g.nz && jr[0] < g.ny, k < g.nz && jr[1] < g.ny};
-    float rho_n[2] = {0.f, 0.f}, q_n[2] = {0.f, 0.f}, h_n[2] = {0.f, 0.f};
-    uint8_t f_n[2] = {0, 0};
-#pragma unroll
-    for (int r = 0; r < 2; ++r)
-        if (rowok[r]) {
-            const int idx = ib * plane + jr[r] * g.nz + k;
-            rho_n[r] = __ldg(&R[idx]);
-            if (c.is_active) q_n[r] = __ldg(&src[idx]);
-            if (MODE == 1) { f_n[r] = __ldg(&F[idx]); h_n[r] = H[idx]; }
-        }
-    bool ok = mbar_wait(&bar[0], 0);
-    ok = mbar_wait(&bar[1], 0) && ok;
-    for (int i = ib; i < ie; ++i) {
-        const int q = i - ib + 1;
-        float rho_c[2], q_c[2], h_c[2];
-        uint8_t f_c[2];
-#pragma unroll
-        for (int r = 0; r < 2; ++r) { rho_c[r] = rho_n[r]; q_c[r] = q_n[r]; h_c[r] = h_n[r]; f_c[r] = f_n[r]; }
-        if (i + 1 < ie) {
-#pragma unroll
-            for (int r = 0; r < 2; ++r)
-                if (rowok[r]) {
-                    const int idx = (i + 1) * plane + jr[r] * g.nz + k;
-                    rho_n[r] = __ldg(&R[idx]);
-                    if (c.is_active) q_n[r] = __ldg(&src[idx]);
-                    if (MODE == 1) { f_n[r] = __ldg(&F[idx]); h_n[r] = H[idx]; }
+    const int i0 = blockIdx.y * g.ni, i1 = min(i0 + g.ni, g.nx);
+    // neighbours outside the grid are read from the voxel itself: no step, no flux
+    const int to_s = j > 0 ? -g.nz : 0, to_n = j + 1 < g.ny ? g.nz : 0;
+    const bool edge_b = gi > 0 && lane == 0, edge_a = gi + 1 < G && (lane == 31 || !on);
+    const bool wall = gi == 0 || gi == G - 1;
+    // The -y face's product enters the sum rounded, or within the multiply-add in rows 8..15 of every
+    // 16 when rows are whole float4s: the rounding that recorded runs of such grids have.
+    const bool fuse = VEC && (j & 8);
+    const float2 ys = fuse ? make_float2(g.idy2, g.idy2) : make_float2(1.0f, 1.0f);
+    int idx = i0 * plane + j * g.nz + z;
+    float4 Tc = load4_ro<VEC>(T + idx, left), Kc = load4_ro<VEC>(K + idx, left);
+    unsigned fl = 0u;
+    if (MODE == 1) fl = load_flags4<VEC>(F + idx, left);
+    float2 fwa, fwb;   // flux through the -x faces, of voxels 0, 1 and 2, 3
+    {
+        const int to_w = i0 > 0 ? -plane : 0;
+        const float4 Tm = load4_ro<VEC>(T + idx + to_w, left), Km = load4_ro<VEC>(K + idx + to_w, left);
+        const float2 m2 = make_float2(2.0f, 2.0f), m1 = make_float2(-1.0f, -1.0f);
+        fwa = scale2(face2(__fmul2_rn(m2, lo2(Kc)), lo2(Kc), lo2(Km), __fmul2_rn(m1, lo2(Tc)), lo2(Tm)), g.idx2);
+        fwb = scale2(face2(__fmul2_rn(m2, hi2(Kc)), hi2(Kc), hi2(Km), __fmul2_rn(m1, hi2(Tc)), hi2(Tm)), g.idx2);
+    }
+    for (int i = i0; i < i1; ++i, idx += plane) {
+        // all of this plane's loads first; the flags were loaded a plane ahead, so that the source and
+        // the enthalpy are read only where they are used
+        const unsigned f4 = fl;
+        const int to_e = i + 1 < g.nx ? plane : 0;
+        const float4 Te = load4_ro<VEC>(T + idx + to_e, left), Ke = load4_ro<VEC>(K + idx + to_e, left);
+        const float4 Ts = load4_ro<VEC>(T + idx + to_s, left), Ks = load4_ro<VEC>(K + idx + to_s, left);
+        const float4 Tq = load4_ro<VEC>(T + idx + to_n, left), Kq = load4_ro<VEC>(K + idx + to_n, left);
+        const float4 rho = load4_ro<VEC>(R + idx, left);
+        float4 sr = make_float4(0.f, 0.f, 0.f, 0.f), h4 = sr;
+        if (c.is_active && (MODE == 0 || !c.zero_src_in_ablated || (f4 & 0x01010101u) != 0x01010101u))
+            sr = load4_ro<VEC>(src + idx, left);
+        if (MODE == 1 && ((f4 | (f4 >> 1)) & 0x01010101u) != 0x01010101u) h4 = load4<VEC>(H + idx, left);
+        if (MODE == 1 && i + 1 < i1) fl = load_flags4<VEC>(F + idx + plane, left);
+        const unsigned dry4 = MODE == 1 && CHAR && on ? (f4 >> 1) & ~f4 & 0x01010101u : 0u;
+        float4 x4 = make_float4(0.f, 0.f, 0.f, 0.f), o4 = x4;
+        if (MODE == 1 && CHAR && dry4) x4 = load4<VEC>(Chi + idx, left);
+        if (MODE == 1 && ARR && on && (f4 & 0x01010101u) != 0x01010101u) o4 = load4<VEC>(Om + idx, left);
+        float Tb = 0.f, Kb = 0.f, Ta = 0.f, Ka = 0.f;
+        if (edge_b) { Tb = __ldg(T + idx - 1); Kb = __ldg(K + idx - 1); }
+        if (edge_a) { Ta = __ldg(T + idx + 4); Ka = __ldg(K + idx + 4); }
+        const float2 k2a = __fmul2_rn(make_float2(2.0f, 2.0f), lo2(Kc)), k2b = __fmul2_rn(make_float2(2.0f, 2.0f), hi2(Kc));
+        const float2 nta = __fmul2_rn(make_float2(-1.0f, -1.0f), lo2(Tc)), ntb = __fmul2_rn(make_float2(-1.0f, -1.0f), hi2(Tc));
+        // z faces: f[v] between voxel v and v + 1, the lower one of voxel 0 from the lane below
+        const float Tu = __shfl_down_sync(0xffffffffu, Tc.x, 1), Ku = __shfl_down_sync(0xffffffffu, Kc.x, 1);
+        if (!edge_a) { Ta = Tu; Ka = Ku; }
+        float fz0 = __fmul_rn(face(k2a.x, Kc.x, Kc.y, nta.x, Tc.y), g.idz2);
+        float fz1 = __fmul_rn(face(k2a.y, Kc.y, Kc.z, nta.y, Tc.z), g.idz2);
+        float fz2 = __fmul_rn(face(k2b.x, Kc.z, Kc.w, ntb.x, Tc.w), g.idz2);
+        float fz3 = __fmul_rn(face(k2b.y, Kc.w, Ka, ntb.y, Ta), g.idz2);
+        float fzb = -__shfl_up_sync(0xffffffffu, fz3, 1);
+        if (edge_b) fzb = __fmul_rn(face(k2a.x, Kc.x, Kb, nta.x, Tb), g.idz2);
+        float lo1 = -fz0, lo2_ = -fz1, lo3 = -fz2;
+        if (wall) {
+            // the row's first and last voxel lose heat through their z faces instead
+            const int last = left - 1;
+            const float Tw = gi == 0 ? Tc.x : (VEC || last == 3 ? Tc.w : last == 2 ? Tc.z : last == 1 ? Tc.y : Tc.x);
+            const float kw = gi == 0 ? Kc.x : (VEC || last == 3 ? Kc.w : last == 2 ? Kc.z : last == 1 ? Kc.y : Kc.x);
+            const float fl0 = zwall_flux<BC>(Tw, kw, g);
+            if (gi == 0) fzb = fl0;
+            if (gi == G - 1) {
+                float up = fl0;
+                if (G == 1) {
+                    const float Tl = last == 3 ? Tc.w : last == 2 ? Tc.z : last == 1 ? Tc.y : Tc.x;
+                    const float kl = last == 3 ? Kc.w : last == 2 ? Kc.z : last == 1 ? Kc.y : Kc.x;
+                    up = zwall_flux<BC>(Tl, kl, g);
                 }
+                if (VEC || last == 3) fz3 = up;
+                else if (last == 2) fz2 = up;
+                else if (last == 1) fz1 = up;
+                else fz0 = up;
+            }
         }
-        ok = mbar_wait(&bar[(q + 1) % ST_STAGES], ((q + 1) / ST_STAGES) & 1) && ok;
-        const float* Tm = ringT[(q - 1) % ST_STAGES];
-        const float* Tc_ = ringT[q % ST_STAGES];
-        const float* Tp = ringT[(q + 1) % ST_STAGES];
-        const float* Km = ringK[(q - 1) % ST_STAGES];
-        const float* Kc = ringK[q % ST_STAGES];
-        const float* Kp = ringK[(q + 1) % ST_STAGES];
+        const float2 fea = scale2(face2(k2a, lo2(Kc), lo2(Ke), nta, lo2(Te)), g.idx2);
+        const float2 feb = scale2(face2(k2b, hi2(Kc), hi2(Ke), ntb, hi2(Te)), g.idx2);
+        float2 da = __fadd2_rn(fwa, fea), db = __fadd2_rn(fwb, feb);
+        fwa = make_float2(-fea.x, -fea.y);
+        fwb = make_float2(-feb.x, -feb.y);
+        float2 sa = face2(k2a, lo2(Kc), lo2(Ks), nta, lo2(Ts)), sb = face2(k2b, hi2(Kc), hi2(Ks), ntb, hi2(Ts));
+        if (!fuse) { sa = scale2(sa, g.idy2); sb = scale2(sb, g.idy2); }
+        da = __ffma2_rn(sa, ys, da);
+        db = __ffma2_rn(sb, ys, db);
+        da = __fadd2_rn(da, scale2(face2(k2a, lo2(Kc), lo2(Kq), nta, lo2(Tq)), g.idy2));
+        db = __fadd2_rn(db, scale2(face2(k2b, hi2(Kc), hi2(Kq), ntb, hi2(Tq)), g.idy2));
+        da = __fadd2_rn(__fadd2_rn(da, make_float2(fzb, lo1)), make_float2(fz0, fz1));
+        db = __fadd2_rn(__fadd2_rn(db, make_float2(lo2_, lo3)), make_float2(fz2, fz3));
+        float2 qa = scale2(lo2(sr), c.q_scale), qb = scale2(hi2(sr), c.q_scale);
+        if (MODE == 1 && c.zero_src_in_ablated && (f4 & 0x01010101u)) {
+            if (f4 & 0x00000001u) qa.x = 0.0f;
+            if (f4 & 0x00000100u) qa.y = 0.0f;
+            if (f4 & 0x00010000u) qb.x = 0.0f;
+            if (f4 & 0x01000000u) qb.y = 0.0f;
+        }
+        const float2 dt2 = make_float2(g.dt, g.dt);
+        const float2 ra = rcp_approx2(make_float2(fmaxf(rho.x, 1e-12f), fmaxf(rho.y, 1e-12f)));
+        const float2 rb = rcp_approx2(make_float2(fmaxf(rho.z, 1e-12f), fmaxf(rho.w, 1e-12f)));
+        const float2 ta = __ffma2_rn(__fmul2_rn(dt2, __fadd2_rn(da, qa)), ra, lo2(Tc));
+        const float2 tb = __ffma2_rn(__fmul2_rn(dt2, __fadd2_rn(db, qb)), rb, hi2(Tc));
+        float out[4] = {ta.x, ta.y, tb.x, tb.y};
+        if (MODE == 1) {
+            float h[4] = {h4.x, h4.y, h4.z, h4.w};
+            const float rh[4] = {rho.x, rho.y, rho.z, rho.w};
+            const unsigned abl4 = f4 & 0x01010101u, dead4 = (f4 | (f4 >> 1)) & 0x01010101u;
+            bool boils = false;   // a wet voxel above the plateau, or with enthalpy banked
+            if (abl4) {
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            if (!rowok[r]) continue;
-            const int j = jr[r];
-            const int jy = j - j0;
-            const int idx = i * plane + j * g.nz + k;
-            const int t = (jy + 1) * ST_PZ + threadIdx.x + 4;
-            const float Tc = Tc_[t], kc = Kc[t];
-            const float fw = (i > 0) ? kface(kc, Km[t]) * (Tm[t] - Tc) * g.idx2 : 0.0f;
-            const float fe = (i + 1 < g.nx) ? kface(kc, Kp[t]) * (Tp[t] - Tc) * g.idx2 : 0.0f;
-            const float fs = (j > 0) ? kface(kc, Kc[t - ST_PZ]) * (Tc_[t - ST_PZ] - Tc) * g.idy2 : 0.0f;
-            const float fn = (j + 1 < g.ny) ? kface(kc, Kc[t + ST_PZ]) * (Tc_[t + ST_PZ] - Tc) * g.idy2 : 0.0f;
-            const float ft = (k > 0) ? kface(kc, Kc[t - 1]) * (Tc_[t - 1] - Tc) * g.idz2 : zwall_flux<BC>(Tc, kc, g);
-            const float fb = (k + 1 < g.nz) ? kface(kc, Kc[t + 1]) * (Tc_[t + 1] - Tc) * g.idz2
-                                            : zwall_flux<BC>(Tc, kc, g);
-            const float div = fw + fe + fs + fn + ft + fb;
-            const float rho = rho_c[r];
-            const float cap = fmaxf(rho, 1e-12f);
-            const uint8_t f = f_c[r];
-            float qv = q_c[r] * c.q_scale;
-            if (MODE == 1 && c.zero_src_in_ablated && (f & BD_FLAG_ABLATED)) qv = 0.0f;
-            if (!c.is_active) qv = 0.0f;
-            float Tt = Tc + __fdividef(g.dt * (div + qv), cap);
-            if (MODE == 1) {
-                const bool abl = (f & BD_FLAG_ABLATED) != 0;
-                const bool dry = (f & BD_FLAG_DRY) != 0;
-                if (abl) {
-                    if (Tt > c.t_void) Tt = c.t_void;
-                } else if (!dry) {
-                    const float h = h_c[r];
-                    if (Tt > c.t_abl) {
-                        H[idx] = h + (Tt - c.t_abl) * rho;
-                        Tt = c.t_abl;
-                    } else if (h > 0.0f) {
-                        const float rel = fminf(h, (c.t_abl - Tt) * rho);
-                        H[idx] = h - rel;
-                        Tt = Tt + rel / rho;
+                for (int v = 0; v < 4; ++v)
+                    if (((f4 >> (8 * v)) & BD_FLAG_ABLATED) && out[v] > c.t_void) out[v] = c.t_void;
+            }
+            if (dead4 != 0x01010101u) {
+#pragma unroll
+                for (int v = 0; v < 4; ++v)
+                    boils |= !((f4 >> (8 * v)) & (BD_FLAG_ABLATED | BD_FLAG_DRY)) && (out[v] > c.t_abl || h[v] > 0.0f);
+            }
+            if (boils && on) {
+#pragma unroll
+                for (int v = 0; v < 4; ++v) {
+                    if ((f4 >> (8 * v)) & (BD_FLAG_ABLATED | BD_FLAG_DRY)) continue;
+                    if (out[v] > c.t_abl) {
+                        h[v] = h[v] + (out[v] - c.t_abl) * rh[v];
+                        out[v] = c.t_abl;
+                    } else if (h[v] > 0.0f) {
+                        const float rel = fminf(h[v], (c.t_abl - out[v]) * rh[v]);
+                        h[v] = h[v] - rel;
+                        out[v] = out[v] + rel / rh[v];
                     }
                 }
-                if (ARR && !abl) Om[idx] += g.dt * c.arr_A * expf(-c.arr_EaR / (Tt + 273.15f));
-                if (CHAR && dry && !abl) {
-                    const float rate = c.char_A * expf(-c.char_EaR / (Tt + 273.15f));
-                    const float x = Chi[idx];
-                    Chi[idx] = 1.0f - (1.0f - x) * expf(-rate * g.dt);
+                store4<VEC>(H + idx, h, left);
+            }
+            if (ARR && on && (f4 & 0x01010101u) != 0x01010101u) {
+                float o[4] = {o4.x, o4.y, o4.z, o4.w};
+#pragma unroll
+                for (int v = 0; v < 4; ++v)
+                    if (!((f4 >> (8 * v)) & BD_FLAG_ABLATED)) o[v] += g.dt * c.arr_A * expf(-c.arr_EaR / (out[v] + 273.15f));
+                store4<VEC>(Om + idx, o, left);
+            }
+            if (CHAR) {
+                const unsigned who = __ballot_sync(0xffffffffu, dry4 != 0u);
+                // below t_cold the rate times dt is under 2^-27, and exp(-rate dt) is 1
+                bool cold = true;
+#pragma unroll
+                for (int v = 0; v < 4; ++v) cold = cold && out[v] > -273.0f && out[v] < c.t_cold;
+                if (who && !__any_sync(0xffffffffu, dry4 && !cold)) {
+                    const float x[4] = {dry4 & 0x00000001u ? 1.0f - (1.0f - x4.x) : x4.x,
+                                        dry4 & 0x00000100u ? 1.0f - (1.0f - x4.y) : x4.y,
+                                        dry4 & 0x00010000u ? 1.0f - (1.0f - x4.z) : x4.z,
+                                        dry4 & 0x01000000u ? 1.0f - (1.0f - x4.w) : x4.w};
+                    if (dry4 && (x[0] != x4.x || x[1] != x4.y || x[2] != x4.z || x[3] != x4.w))
+                        store4<VEC>(Chi + idx, x, left);
+                } else if (who) {
+                    // Two exponentials and a division a voxel, needed by the few dry ones: the warp's dry
+                    // groups pass their voxels to all its lanes, 8 groups at a time (thin dry layers cost
+                    // every warp that crosses one 4 rounds for a handful of lanes otherwise).
+                    const int rank = __popc(who & ((1u << lane) - 1u));
+                    float4* box = work[threadIdx.x >> 5];
+                    for (int k0 = 0; k0 < __popc(who); k0 += 8) {
+                        const int slot = rank - k0;
+                        const bool mine = dry4 && slot >= 0 && slot < 8;
+                        if (mine) {
+                            box[slot] = make_float4(out[0], out[1], out[2], out[3]);
+                            box[8 + slot] = x4;
+                        }
+                        __syncwarp();
+                        const float Tv = reinterpret_cast<const float*>(box)[lane];
+                        float* xp = reinterpret_cast<float*>(box + 8) + lane;
+                        if (k0 + (lane >> 2) < __popc(who)) {
+                            const float rate = c.char_A * expf(-c.char_EaR / (Tv + 273.15f));
+                            *xp = 1.0f - (1.0f - *xp) * expf(-rate * g.dt);
+                        }
+                        __syncwarp();
+                        if (mine) {
+                            const float4 y = box[8 + slot];
+                            const float x[4] = {dry4 & 0x00000001u ? y.x : x4.x, dry4 & 0x00000100u ? y.y : x4.y,
+                                                dry4 & 0x00010000u ? y.z : x4.z, dry4 & 0x01000000u ? y.w : x4.w};
+                            store4<VEC>(Chi + idx, x, left);
+                        }
+                        __syncwarp();
+                    }
                 }
             }
-            Tn[idx] = Tt;
         }
-        __syncthreads();  // every thread is done with plane i-1's stage
-        if (tid == 0 && q + 3 < nplanes) {
-            const int s = (q + 3) % ST_STAGES;
-            fence_proxy_async_smem();
-            mbar_expect_tx(&bar[s], 2 * ST_TILE_BYTES);
-            tma_load_3d(ringT[s], &t_map, k0 - 4, j0 - 1, i + 3, &bar[s]);
-            tma_load_3d(ringK[s], &k_map, k0 - 4, j0 - 1, i + 3, &bar[s]);
-        }
-    }
-    if (!ok) {
-        atomicExch(err, 1);
-        for (int q = 0; q < ST_STAGES; ++q) {
-            const int last = nplanes - 1 - ((nplanes - 1 - q) % ST_STAGES + ST_STAGES) % ST_STAGES;
-            if (last >= 0) mbar_wait(&bar[q], (last / ST_STAGES) & 1);
-        }
+        if (on) store4<VEC>(Tn + idx, out, left);
+        Tc = Te;
+        Kc = Ke;
     }
 }
 
@@ -284,28 +328,10 @@ __global__ void k_pack_flags(const uint8_t* __restrict__ abl, const uint8_t* __r
     }
 }
 
-static dim3 tile_grid(int nx, int ny, int nz, int ni) {
-    return dim3((nz + TZ - 1) / TZ, (ny + TY - 1) / TY, (nx + ni - 1) / ni);
-}
-
-static int pick_ni(int nx, int ny, int nz) {
-    // short marches (~8 planes) and several waves of 256-thread CTAs: enough independent
-    // DRAM round trips in flight to cover latency without a long serial chain per thread
-    long long cols = (long long)((nz + TZ - 1) / TZ) * ((ny + TY - 1) / TY);
-    long long want = 148LL * 6 * 4;
-    long long chunks = std::max(1LL, want / std::max(1LL, cols));
-    int ni = (int)std::max(4LL, ((long long)nx + chunks - 1) / chunks);
-#ifndef BD_STENCIL_NI
-#define BD_STENCIL_NI 8
-#endif
-    ni = std::min(ni, BD_STENCIL_NI);
-    return std::min(ni, std::max(nx, 1));
-}
-
 static Geo make_geo(int nx, int ny, int nz, float dx, float dy, float dz, float dt, float h, float tamb) {
     Geo g;
     g.nx = nx; g.ny = ny; g.nz = nz;
-    g.ni = pick_ni(nx, ny, nz);
+    g.ni = 1;
     g.idx2 = 1.0f / (dx * dx); g.idy2 = 1.0f / (dy * dy); g.idz2 = 1.0f / (dz * dz);
     g.dz = dz; g.h_eff = h; g.t_amb = tamb; g.dt = dt;
     return g;
@@ -330,54 +356,43 @@ static size_t substep_pad_bytes(int cap, const void* kernel) {
     return (size_t)pad;
 }
 
+// x planes per CTA: the knob's, fewer where that leaves the chip idle (a CTA of few planes reads its
+// halo planes of T and k for fewer of its own). Aiming at 12 CTAs per SM: 150x150x138 0.64 ms per 20
+// substeps against 0.69 - 0.74 at 6, 24 and 48; 200x200x192 takes the knob's 8 planes either way.
+static int substep_planes(int tiles, int nx) {
+    const int want = std::max(1, 148 * SUB_WAVE / std::max(1, tiles));   // chunks that fill the chip
+    const int ni = std::max(1, std::min(tune_value(BD_TUNE_STENCIL_XC), nx / std::min(want, nx)));
+    return std::max(ni, (nx + 65534) / 65535);   // chunks fit the grid's second dimension
+}
+
 template <int MODE, int BC, bool ARR, bool CHAR>
 static void launch_substeps(const Geo& g, const AblConst& c, float* Ta, float* Tb, int n, const float* src,
                             const float* K, const float* R, const uint8_t* F, float* H, float* Om, float* Chi,
-                            cudaStream_t st, int* err) {
-    CUtensorMap ma, mb, mk;
-#ifdef BD_NO_TMA
-    err = nullptr;
-#endif
-    const bool tma = err != nullptr && make_tmap_3d_f32(&ma, Ta, g.nx, g.ny, g.nz, ST_PZ, ST_PY, 1) &&
-                     make_tmap_3d_f32(&mb, Tb, g.nx, g.ny, g.nz, ST_PZ, ST_PY, 1) &&
-                     make_tmap_3d_f32(&mk, K, g.nx, g.ny, g.nz, ST_PZ, ST_PY, 1);
-    if (tma) {
-        const int xc = tune_value(BD_TUNE_STENCIL_XC);
-        const dim3 grid((g.nz + ST_BZ - 1) / ST_BZ, (g.ny + ST_BY - 1) / ST_BY, (g.nx + xc - 1) / xc);
-        const size_t pad = substep_pad_bytes(tune_value(BD_TUNE_STENCIL_CAP), (const void*)k_substep_tma<MODE, BC, ARR, CHAR>);
-        for (int s = 0; s < n; ++s) {
-            float* out = (s & 1) ? Ta : Tb;
-            k_substep_tma<MODE, BC, ARR, CHAR><<<grid, dim3(TZ, TY), pad, st>>>((s & 1) ? mb : ma, mk, g, c, out, src,
-                                                                               R, F, H, Om, Chi, xc, err);
-        }
-        return;
-    }
-    dim3 grid = tile_grid(g.nx, g.ny, g.nz, g.ni), block(TZ, TY);
-    for (int s = 0; s < n; ++s) {
-        const float* in = (s & 1) ? Tb : Ta;
-        float* out = (s & 1) ? Ta : Tb;
-        k_substep<MODE, BC, ARR, CHAR><<<grid, block, 0, st>>>(g, c, in, out, src, K, R, F, H, Om, Chi);
-    }
+                            cudaStream_t st) {
+    Geo gg = g;
+    const int groups = (g.nz + 3) / 4 * g.ny;
+    const int tiles = (groups + SUB_T - 1) / SUB_T;
+    gg.ni = substep_planes(tiles, g.nx);
+    const dim3 grid(tiles, (g.nx + gg.ni - 1) / gg.ni);
+    const uintptr_t bits = (uintptr_t)Ta | (uintptr_t)Tb | (uintptr_t)src | (uintptr_t)K | (uintptr_t)R | (uintptr_t)H |
+                           (uintptr_t)Om | (uintptr_t)Chi;
+    const bool vec = g.nz % 4 == 0 && (bits & 15) == 0 && ((uintptr_t)F & 3) == 0;
+    auto run = [&](auto v) {
+        constexpr bool VEC = decltype(v)::value;
+        const size_t pad = substep_pad_bytes(tune_value(BD_TUNE_STENCIL_CAP), (const void*)k_substep<MODE, BC, ARR, CHAR, VEC>);
+        for (int s = 0; s < n; ++s)
+            k_substep<MODE, BC, ARR, CHAR, VEC><<<grid, SUB_T, pad, st>>>(gg, c, (s & 1) ? Tb : Ta, (s & 1) ? Ta : Tb, src,
+                                                                          K, R, F, H, Om, Chi);
+    };
+    if (vec) run(std::true_type{});
+    else run(std::false_type{});
 }
 
-// Runs `launch(err)` with a 4-byte device error flag, then synchronises the stream and turns a
-// raised flag (a bounded TMA wait that timed out) into BD_ERR_TIMEOUT.
-template <typename F>
-static int with_error_flag(cudaStream_t st, const char* what, F launch) {
-    int* err = nullptr;
-    BD_CUDA(scratch_alloc((void**)&err, sizeof(int), st));
-    int rc = BD_OK;
-    int host_err = 0;
-    cudaError_t e = cudaMemsetAsync(err, 0, sizeof(int), st);
-    if (e == cudaSuccess) rc = launch(err);
-    if (e == cudaSuccess && rc == BD_OK) e = cudaMemcpyAsync(&host_err, err, sizeof(int), cudaMemcpyDeviceToHost, st);
-    cudaError_t e2 = cudaFreeAsync(err, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+// The synchronous entry points' end: waits for the launches and reports what went wrong in them.
+static int finish(int rc, cudaStream_t st, const char* what) {
     if (rc) return rc;
-    if (e != cudaSuccess) return cuda_status(e, what);
-    if (e2 != cudaSuccess) return cuda_status(e2, what);
-    if (host_err) return fail(BD_ERR_TIMEOUT, "%s: a bounded TMA wait timed out", what);
-    return BD_OK;
+    const cudaError_t e = cudaStreamSynchronize(st);
+    return e == cudaSuccess ? BD_OK : cuda_status(e, what);
 }
 
 }  // namespace bd
@@ -399,30 +414,36 @@ extern "C" int bd_thermal_advance(const BdThermalParams* p, float* Ta, float* Tb
     c.q_scale = p->q_scale;
     c.is_active = p->is_active;
     cudaStream_t st = as_stream(stream);
-    return with_error_flag(st, "bd_thermal_advance", [&](int* err) -> int {
-        if (p->bc_mode == BD_BC_SERIES)
-            launch_substeps<0, BD_BC_SERIES, false, false>(g, c, Ta, Tb, n, src, K, R, nullptr, nullptr, nullptr,
-                                                           nullptr, st, err);
-        else
-            launch_substeps<0, BD_BC_METAL, false, false>(g, c, Ta, Tb, n, src, K, R, nullptr, nullptr, nullptr,
-                                                          nullptr, st, err);
-        BD_CHECK_LAUNCH("k_substep<thermal>");
-        return BD_OK;
-    });
+    if (p->bc_mode == BD_BC_SERIES)
+        launch_substeps<0, BD_BC_SERIES, false, false>(g, c, Ta, Tb, n, src, K, R, nullptr, nullptr, nullptr, nullptr, st);
+    else
+        launch_substeps<0, BD_BC_METAL, false, false>(g, c, Ta, Tb, n, src, K, R, nullptr, nullptr, nullptr, nullptr, st);
+    BD_CHECK_LAUNCH("k_substep<thermal>");
+    return finish(BD_OK, st, "bd_thermal_advance");
 }
 
 namespace bd {
+// The temperature (degC) up to which A exp(-E / T) dt stays below 2^-27: T = E / ln(A dt 2^27), a tenth of a
+// kelvin lower for the rounding of the kernel's own evaluation. Nowhere (-inf) unless A, E, dt > 0.
+static float char_cold_limit(double A, double E, double dt) {
+    const double x = A * dt * 134217728.0;
+    if (!(A > 0.0) || !(E > 0.0) || !(dt > 0.0) || !std::isfinite(x) || !std::isfinite(E)) return -INFINITY;
+    if (x <= 1.0) return -INFINITY;   // below the limit at any temperature: rare enough for the general path
+    return (float)(E / std::log(x) - 273.15 - 0.1);
+}
+
 int ablation_launch(const BdAblationParams* p, float* Ta, float* Tb, int n, float* H, float* Om, float* Chi,
-                    const uint8_t* F, const float* src, const float* K, const float* R, cudaStream_t st, int* err) {
+                    const uint8_t* F, const float* src, const float* K, const float* R, cudaStream_t st) {
     Geo g = make_geo(p->nx, p->ny, p->nz, p->dx, p->dy, p->dz, p->dt, p->h_eff, p->t_ambient);
     AblConst c;
     c.t_abl = p->t_abl; c.t_void = p->t_void; c.q_scale = p->q_scale;
     c.arr_A = p->arr_A; c.arr_EaR = p->arr_Ea_over_R; c.char_A = p->char_A; c.char_EaR = p->char_Ea_over_R;
     c.zero_src_in_ablated = p->zero_src_in_ablated; c.is_active = p->is_active;
+    c.t_cold = p->has_char ? char_cold_limit(p->char_A, p->char_Ea_over_R, p->dt) : 0.0f;
     const bool arr = p->has_arrhenius != 0, chr = p->has_char != 0;
 #define BD_ABL_CASE(BCV, A_, C_)                                                                 \
     if (p->bc_mode == BCV && arr == A_ && chr == C_) {                                           \
-        launch_substeps<1, BCV, A_, C_>(g, c, Ta, Tb, n, src, K, R, F, H, Om, Chi, st, err);     \
+        launch_substeps<1, BCV, A_, C_>(g, c, Ta, Tb, n, src, K, R, F, H, Om, Chi, st);          \
         BD_CHECK_LAUNCH("k_substep<ablation>");                                                  \
         return BD_OK;                                                                            \
     }
@@ -453,9 +474,7 @@ extern "C" int bd_ablation_advance(const BdAblationParams* p, float* Ta, float* 
     BD_REQUIRE((long long)p->nx * p->ny * p->nz < (1LL << 31), "bd_ablation_advance: grid exceeds 2^31 voxels");
     if (n == 0) return BD_OK;
     cudaStream_t st = as_stream(stream);
-    return with_error_flag(st, "bd_ablation_advance", [&](int* err) -> int {
-        return ablation_launch(p, Ta, Tb, n, H, Om, Chi, F, src, K, R, st, err);
-    });
+    return finish(ablation_launch(p, Ta, Tb, n, H, Om, Chi, F, src, K, R, st), st, "bd_ablation_advance");
 }
 
 extern "C" int bd_pack_flags(const uint8_t* abl, const uint8_t* dry, const uint8_t* vd, int64_t n, uint8_t* out,

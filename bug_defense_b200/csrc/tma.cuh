@@ -1,9 +1,6 @@
-// Tensor Memory Accelerator (TMA) helpers for the plane-streaming stencils: host-side tensor-map
-// encoding for C-order (nx, ny, nz) float grids and device-side mbarrier / bulk-tensor copies.
+// mbarrier helpers of the kernels fed by asynchronous bulk copies.
 // Every wait is bounded: after TMA_SPIN_LIMIT polls it raises an error flag instead of hanging.
 #pragma once
-
-#include <cuda.h>
 
 #include "common.cuh"
 
@@ -13,13 +10,6 @@ namespace bd {
 // phase completes), so TMA_SPIN_LIMIT polls bound a wait to about 4 s before it reports a timeout.
 constexpr unsigned TMA_SPIN_LIMIT = 1u << 22;
 constexpr unsigned TMA_SUSPEND_NS = 1000;
-
-// 3-D tiled map over a float grid: dims (innermost first) {nz, ny, nx}; box {bz, by, bx}.
-// Requires nz % 4 == 0 (16-byte row stride) and a 16-byte aligned base; returns false otherwise.
-bool make_tmap_3d_f32(CUtensorMap* out, const void* base, int nx, int ny, int nz, int bz, int by, int bx);
-// 3-D tiled map over a byte grid whose z rows are `pitch` bytes apart (pitch % 16 == 0, >= nz);
-// elements past nz read as 0.
-bool make_tmap_3d_u8(CUtensorMap* out, const void* base, int nx, int ny, int nz, int pitch, int bz, int by, int bx);
 
 __device__ __forceinline__ unsigned smem_addr(const void* p) {
     return static_cast<unsigned>(__cvta_generic_to_shared(p));
@@ -69,16 +59,6 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned pari
 // (TMA) writes to the same buffer.
 __device__ __forceinline__ void fence_proxy_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
-// 3-D tile load into shared memory; c0 (innermost) must keep c0 * 4 bytes 16-byte aligned.
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int c0, int c1, int c2,
-                                            unsigned long long* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
-        "[%5];" ::"r"(smem_addr(dst)),
-        "l"(reinterpret_cast<unsigned long long>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(smem_addr(bar))
-        : "memory");
 }
 
 }  // namespace bd
