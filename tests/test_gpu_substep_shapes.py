@@ -48,5 +48,5 @@ def test_char_of_scattered_dry_voxels(gpu, shape, dry_share):
     want = np.where(dry, 1.0 - (1.0 - chi0) * np.exp(-n * dt * A * np.exp(-E / (T0 + 273.15))), chi0)
     assert np.max(np.abs(chi - want)) <= n * 2.0 ** -24 + 1e-5
     assert np.array_equal(chi[~dry], chi0[~dry])
-    if dry.sum() > 50:                     # the draw holds hot dry voxels
-        assert np.any(want - chi0 > 0.01)
+    if dry.sum() > 50:                     # the draw holds dry voxels that char (1.7e-3 at 600 C)
+        assert np.any(want - chi0 > 1e-4)
