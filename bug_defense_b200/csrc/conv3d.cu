@@ -19,11 +19,16 @@
 // drain the double-buffered accumulators and run the fused epilogue (bias, ReLU, nearest
 // upsampling with the skip add, gradient gating, the 1x1 head).
 //
-// Weight-gradient kernel (k_conv_wgrad): dW[t][co][ci] = sum_v g[v - off_t][co] x[v][ci]. Taps are
-// stacked along M (128/cout taps per MMA): 64-row plane chunks of the shifted gradient are the
-// MN-major, no-swizzle A operand (8 channels per 1 KB core-matrix column) and the activation chunks
-// are MN-major B; each CTA reduces a contiguous range of 64-voxel chunks in TMEM and adds its
-// partial weights with FP32 atomics.
+// Weight-gradient kernel (k_conv_wgrad): dW[(dx, dy), dz][co][ci] = sum_u g[u - (dx, dy)][co] x[u + dz][ci].
+// The nine (dx, dy)-shifted gradient tiles are stacked along M (128/cout pairs per MMA) and the three
+// z-shifted activation tiles along N, so a stage of 64 or 128 rows is loaded once, 9 + 3 tiles, for all
+// 27 taps; plane chunks are the MN-major, no-swizzle operands as they lie (8 channels per core-matrix
+// column). Each CTA reduces a contiguous range of rows in TMEM and adds its partial weights with FP32
+// atomics. Bound by the L2 reads of the shifted tiles. Stacking taps along M only, 27 shifted tiles
+// were loaded in rows of 64, and the activations again for each MMA: 3 times the bytes in copies of
+// 1 KB by one thread. 16 -> 16 channels at 200x200x128: 2.0 ms before, 0.33 ms now (0.38 with one
+// thread issuing the copies); 64 -> 64 at 50x50x32: 0.4 ms before, 0.18; a training step of a
+// 200x200x128 volume 12.1 ms before, 4.7 ms.
 //
 // Every mbarrier wait is bounded; a timeout sets the error flag, the roles drain what they issued
 // and the CTA frees its TMEM and returns.
@@ -44,7 +49,6 @@ namespace {
 constexpr int kTileM = 128;
 constexpr int kPlaneBytes = kTileM * 16;   // one 8-channel plane of a tile: 128 rows x 16 B
 constexpr int kSmemLimit = 232448;     // 227 KB opt-in dynamic shared memory per CTA
-constexpr int kWgradKv = 64;           // voxels per weight-gradient K chunk
 constexpr int kRowMargin = 256;        // zero rows after the padded volume (tile copies overrun it)
 constexpr int kEpiGroups = 2;          // epilogue warp groups (4 warps each), one per accumulator
 constexpr int kConvThreads = 64 + kEpiGroups * 128;
@@ -67,15 +71,6 @@ __host__ __device__ inline Geom make_geom(int nx, int ny, int nz) {
 }
 
 __device__ __forceinline__ size_t prow(const Geom& g, int chunk, int v) { return ((size_t)chunk * g.R + v) * 8; }
-
-__device__ __forceinline__ int tap_offset(const Geom& g, int t, int taps) {
-    if (taps == 27) {
-        const int dx = t / 9 - 1, dy = (t / 3) % 3 - 1, dz = t % 3 - 1;
-        return dx * g.plane + dy * g.nzp + dz;
-    }
-    const int dx = t / 3 - 1, dy = t % 3 - 1;
-    return dx * g.plane + dy * g.nzp;
-}
 
 struct ConvArgs {
     Geom g;        // level of the convolution
@@ -147,6 +142,18 @@ __device__ __forceinline__ bool wait_or_abort(unsigned long long* bar, unsigned 
     ctl->abort = 1;
     if (err) atomicExch(err, 1);
     return false;
+}
+
+// A producer warp whose lanes all issue copies, before it fills a stage of `bytes`: false (in every lane)
+// when the kernel gives up.
+__device__ __forceinline__ bool open_stage(unsigned long long* empty, unsigned parity, unsigned long long* full,
+                                           uint32_t bytes, int lane, SharedCtl* ctl, int* err) {
+    int ok = 0;
+    if (lane == 0) {
+        ok = !ctl->abort && wait_or_abort(empty, parity, ctl, err);
+        if (ok) mbar_expect_tx(full, bytes);
+    }
+    return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 
 constexpr int pow2_at_least(int x) { return x <= 32 ? 32 : x <= 64 ? 64 : x <= 128 ? 128 : x <= 256 ? 256 : 512; }
@@ -457,41 +464,48 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(const ConvArgs a) {
 
 struct WgradArgs {
     Geom g;
-    int taps, g0, g1, chunks_total, chunks_per_cta;
+    int taps, u_lo, chunks_total, chunks_per_cta, cin;
     const __nv_bfloat16* grad;
     const __nv_bfloat16* act;
     float* dw;
     int* err;
 };
 
-template <int COUT, int CIN>
+template <int COUT, int CIS>
 struct WgradCfg {
-    static constexpr int TPG = kTileM / COUT;               // taps per group (stacked along M)
-    static constexpr int CHUNK = kWgradKv * 16;             // 64 rows of one 8-channel plane (1 KB)
-    static constexpr int ABOX = (COUT / 8) * CHUNK;         // one tap's gradient tile
-    static constexpr int BBOX = (CIN / 8) * CHUNK;          // activation tile
-    static constexpr int STAGE = TPG * ABOX + BBOX;
+    static constexpr int TPG = kTileM / COUT;               // (dx, dy) pairs per MMA (stacked along M)
+    static constexpr int NG = (9 + TPG - 1) / TPG;          // MMAs over the 9 pairs; the last one overlaps
+    static constexpr int KV = COUT == 16 ? 128 : 64;        // rows per stage
+    static constexpr int CHUNK = KV * 16;                   // KV rows of one 8-channel plane
+    static constexpr int ABOX = (COUT / 8) * CHUNK;         // one pair's gradient tile
+    static constexpr int BBOX = (CIS / 8) * CHUNK;          // one z shift's activation tile
+    static constexpr int STAGE = 9 * ABOX + 3 * BBOX;
     static constexpr int CTL = 1024;
     static constexpr int NST_FIT = (kSmemLimit - 1024 - CTL) / STAGE;
     static constexpr int NST = NST_FIT > 12 ? 12 : NST_FIT;
     static constexpr int SMEM = 1024 + CTL + NST * STAGE;
-    static constexpr int GMAX = (512 / CIN) < 14 ? (512 / CIN) : 14;   // groups per launch (TMEM columns)
+    static constexpr int TMEM_COLS = pow2_at_least(NG * 3 * CIS);
+    static_assert(NST >= 2, "wgrad: not enough shared memory for a 2-stage pipeline");
     static_assert(SMEM <= kSmemLimit, "wgrad: shared memory over the limit");
     static_assert(STAGE % 1024 == 0, "wgrad: stage must keep 1024-byte alignment");
+    static_assert(NG * 3 * CIS <= 512 && 3 * CIS <= 256, "wgrad: accumulators fit TMEM, N fits an MMA");
+    // first pair of MMA gi: the last one starts early enough to hold TPG pairs
+    __host__ __device__ static constexpr int pair0(int gi) { return gi * TPG + TPG <= 9 ? gi * TPG : 9 - TPG; }
 };
 
-template <int COUT, int CIN>
+// Slice blockIdx.y of CIS input channels. See the file comment for the layout.
+template <int COUT, int CIS>
 __global__ void __launch_bounds__(192, 1) k_conv_wgrad(const WgradArgs a) {
-    using C = WgradCfg<COUT, CIN>;
+    using C = WgradCfg<COUT, CIS>;
     extern __shared__ unsigned char smem_raw[];
     const uint32_t base_addr = smem_addr(smem_raw);
     unsigned char* smem = smem_raw + ((1024 - (base_addr & 1023)) & 1023);
     SharedCtl* ctl = reinterpret_cast<SharedCtl*>(smem);
     unsigned char* stages = smem + C::CTL;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int ng = a.g1 - a.g0;
-    uint32_t tcols = 32;
-    while (tcols < (uint32_t)(ng * CIN)) tcols <<= 1;
+    const int kz = a.taps == 27 ? 3 : 1;
+    const int NN = kz * CIS;                         // MMA N: z taps stacked along N
+    const int ci0 = blockIdx.y * CIS;
 
     const int c_begin = blockIdx.x * a.chunks_per_cta;
     const int c_end = min(a.chunks_total, c_begin + a.chunks_per_cta);
@@ -506,70 +520,69 @@ __global__ void __launch_bounds__(192, 1) k_conv_wgrad(const WgradArgs a) {
         ctl->abort = 0;
         mbar_init_fence();
     }
-    if (warp == 1) tmem_alloc(&ctl->tmem, tcols);
+    if (warp == 1) tmem_alloc(&ctl->tmem, C::TMEM_COLS);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = ctl->tmem;
 
     if (warp == 0) {
-        if (lane == 0) {
-            int s = 0;
-            unsigned ph = 0;
-            long long issued = 0;
-            for (int c = c_begin; c < c_end && !ctl->abort; ++c) {
-                const int v0 = a.g.v_lo + c * kWgradKv;
-                for (int gi = a.g0; gi < a.g1; ++gi) {
-                    if (!wait_or_abort(&ctl->empty[s], ph ^ 1, ctl, a.err)) { c = c_end; break; }
-                    unsigned char* st = stages + s * C::STAGE;
-                    mbar_expect_tx(&ctl->full[s], C::STAGE);
-#pragma unroll
-                    for (int j = 0; j < C::TPG; ++j) {
-                        const int t = min(gi * C::TPG + j, a.taps - 1);
-                        const int row = v0 - tap_offset(a.g, t, a.taps);
-#pragma unroll
-                        for (int cb = 0; cb < COUT / 8; ++cb)
-                            bulk_load(st + j * C::ABOX + cb * C::CHUNK, a.grad + prow(a.g, cb, row), C::CHUNK,
-                                      &ctl->full[s]);
-                    }
-#pragma unroll
-                    for (int cb = 0; cb < CIN / 8; ++cb)
-                        bulk_load(st + C::TPG * C::ABOX + cb * C::CHUNK, a.act + prow(a.g, cb, v0), C::CHUNK,
-                                  &ctl->full[s]);
-                    ++issued;
-                    if (++s == C::NST) { s = 0; ph ^= 1; }
+        const uint32_t bytes = 9 * C::ABOX + kz * C::BBOX;
+        constexpr int NA = 9 * (COUT / 8);               // gradient copies of a stage, then the activations'
+        const int n_copies = NA + kz * (CIS / 8);
+        int s = 0;
+        unsigned ph = 0;
+        long long issued = 0;
+        for (int c = c_begin; c < c_end; ++c) {
+            const int u0 = a.u_lo + c * C::KV;
+            if (!open_stage(&ctl->empty[s], ph ^ 1, &ctl->full[s], bytes, lane, ctl, a.err)) break;
+            unsigned char* st = stages + s * C::STAGE;
+            for (int i = lane; i < n_copies; i += 32) {
+                const __nv_bfloat16* from;
+                if (i < NA) {
+                    const int q = i / (COUT / 8), cb = i % (COUT / 8);
+                    from = a.grad + prow(a.g, cb, u0 - (q / 3 - 1) * a.g.plane - (q % 3 - 1) * a.g.nzp);
+                } else {
+                    const int dz = (i - NA) / (CIS / 8), cb = (i - NA) % (CIS / 8);
+                    from = a.act + prow(a.g, ci0 / 8 + cb, u0 + dz - kz / 2);
                 }
+                bulk_load(st + i * C::CHUNK, from, C::CHUNK, &ctl->full[s]);
             }
+            ++issued;
+            if (++s == C::NST) { s = 0; ph ^= 1; }
+        }
+        __syncwarp();
+        if (lane == 0) {
             const long long n_drain = issued < C::NST ? issued : C::NST;
             for (long long i = 0; i < n_drain; ++i) {
                 if (--s < 0) { s = C::NST - 1; ph ^= 1; }
                 mbar_wait(&ctl->full[s], ph);
             }
         }
+        __syncwarp();
     } else if (warp == 1) {
         if (lane == 0) {
             // MN-major, no swizzle: 8 M (or N) elements x 8 K rows per 128-byte core matrix; K groups
-            // 128 B apart (LBO), 8-element M/N blocks one 1 KB chunk apart (SBO)
-            const uint32_t idesc = umma_idesc_bf16(kTileM, CIN, true, true);
+            // 128 B apart (LBO), 8-element M/N blocks one chunk apart (SBO)
+            const uint32_t idesc = umma_idesc_bf16(kTileM, NN, true, true);
             const uint32_t sbase = smem_addr(stages);
             int s = 0;
             unsigned ph = 0;
-            bool ok = true;
-            for (int c = c_begin; ok && c < c_end && !ctl->abort; ++c) {
-                for (int gi = a.g0; gi < a.g1; ++gi) {
-                    if (!wait_or_abort(&ctl->full[s], ph, ctl, a.err)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint32_t st = sbase + s * C::STAGE;
-                    const uint32_t d = tmem + (gi - a.g0) * CIN;
+            for (int c = c_begin; c < c_end && !ctl->abort; ++c) {
+                if (!wait_or_abort(&ctl->full[s], ph, ctl, a.err)) break;
+                tc_fence_after();
+                const uint32_t st = sbase + s * C::STAGE;
 #pragma unroll
-                    for (int kk = 0; kk < kWgradKv / 16; ++kk) {
-                        const uint64_t ad = umma_desc(st + kk * 256, 128, C::CHUNK, UMMA_NONE);
-                        const uint64_t bd = umma_desc(st + C::TPG * C::ABOX + kk * 256, 128, C::CHUNK, UMMA_NONE);
-                        umma_bf16(d, ad, bd, idesc, (c != c_begin) || kk != 0);
+                for (int kk = 0; kk < C::KV / 16; ++kk) {
+                    const uint64_t bd = umma_desc(st + 9 * C::ABOX + kk * 256, 128, C::CHUNK, UMMA_NONE);
+#pragma unroll
+                    for (int gi = 0; gi < C::NG; ++gi) {
+                        const uint64_t ad = umma_desc(st + C::pair0(gi) * C::ABOX + kk * 256, 128, C::CHUNK, UMMA_NONE);
+                        umma_bf16(tmem + gi * NN, ad, bd, idesc, (c != c_begin) || kk != 0);
                     }
-                    umma_commit(&ctl->empty[s]);
-                    if (++s == C::NST) { s = 0; ph ^= 1; }
                 }
+                umma_commit(&ctl->empty[s]);
+                if (++s == C::NST) { s = 0; ph ^= 1; }
             }
             umma_commit(&ctl->acc_full[0]);
             mbar_wait(&ctl->acc_full[0], 0);
@@ -580,17 +593,20 @@ __global__ void __launch_bounds__(192, 1) k_conv_wgrad(const WgradArgs a) {
         if (wait_or_abort(&ctl->acc_full[0], 0, ctl, a.err) && !ctl->abort) {
             tc_fence_after();
             const int j = row / COUT, co = row % COUT;
-            for (int gi = a.g0; gi < a.g1; ++gi) {
-                float v[CIN];
+            for (int gi = 0; gi < C::NG; ++gi) {
+                const int q = C::pair0(gi) + j;
+                const bool mine = q >= gi * C::TPG;      // not already the MMA before's
+                for (int dz = 0; dz < kz; ++dz) {
+                    float v[CIS];
 #pragma unroll
-                for (int c = 0; c < CIN; c += 16)
-                    tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (gi - a.g0) * CIN + c, v + c);
-                tmem_ld_wait();
-                const int t = gi * C::TPG + j;
-                if (t < a.taps) {
-                    float* dst = a.dw + ((size_t)t * COUT + co) * CIN;
+                    for (int c = 0; c < CIS; c += 16)
+                        tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + gi * NN + dz * CIS + c, v + c);
+                    tmem_ld_wait();
+                    if (mine) {
+                        float* dst = a.dw + ((size_t)(q * kz + dz) * COUT + co) * a.cin + ci0;
 #pragma unroll
-                    for (int c = 0; c < CIN; ++c) atomicAdd(dst + c, v[c]);
+                        for (int c = 0; c < CIS; ++c) atomicAdd(dst + c, v[c]);
+                    }
                 }
             }
         }
@@ -599,7 +615,7 @@ __global__ void __launch_bounds__(192, 1) k_conv_wgrad(const WgradArgs a) {
     __syncthreads();
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem, tcols);
+        tmem_dealloc(tmem, C::TMEM_COLS);
     }
 }
 
@@ -659,30 +675,30 @@ int launch_conv_t(const BdConvCall& c, cudaStream_t st, int* err, int sms) {
     return BD_OK;
 }
 
-template <int COUT, int CIN>
-int launch_wgrad_t(int nx, int ny, int nz, int taps, const void* grad, const void* act, float* dw, cudaStream_t st,
-                   int* err, int sms) {
-    using C = WgradCfg<COUT, CIN>;
-    BD_CUDA(cudaFuncSetAttribute(k_conv_wgrad<COUT, CIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
+template <int COUT, int CIS>
+int launch_wgrad_t(int nx, int ny, int nz, int cin, int taps, const void* grad, const void* act, float* dw,
+                   cudaStream_t st, int* err, int sms) {
+    using C = WgradCfg<COUT, CIS>;
+    BD_CUDA(cudaFuncSetAttribute(k_conv_wgrad<COUT, CIS>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
     WgradArgs a{};
     a.g = make_geom(nx, ny, nz);
     a.taps = taps;
-    a.chunks_total = (a.g.v_hi - a.g.v_lo + kWgradKv - 1) / kWgradKv;
+    a.cin = cin;
+    // rows u of the sums g[u - (dx, dy)] x[u + dz]: one more on either side than the interior has
+    a.u_lo = a.g.v_lo - 1;
+    a.chunks_total = (a.g.v_hi + 1 - a.u_lo + C::KV - 1) / C::KV;
     a.grad = static_cast<const __nv_bfloat16*>(grad);
     a.act = static_cast<const __nv_bfloat16*>(act);
     a.dw = dw;
     a.err = err;
-    const int groups = (taps + C::TPG - 1) / C::TPG;
-    // split the voxels over the SMs; small levels keep at least 32 chunks per CTA
-    const int ctas = std::max(1, std::min(sms, (a.chunks_total + 31) / 32));
+    // split the rows over the SMs; small levels keep at least 2048 rows per CTA (a CTA ends by adding
+    // its 27 x cout x CIS partial weights to memory)
+    const int slices = cin / CIS;
+    const int ctas = std::max(1, std::min(std::max(1, sms / slices), (a.chunks_total * C::KV + 2047) / 2048));
     a.chunks_per_cta = (a.chunks_total + ctas - 1) / ctas;
     const int grid = (a.chunks_total + a.chunks_per_cta - 1) / a.chunks_per_cta;
-    for (int g0 = 0; g0 < groups; g0 += C::GMAX) {
-        a.g0 = g0;
-        a.g1 = std::min(groups, g0 + C::GMAX);
-        k_conv_wgrad<COUT, CIN><<<grid, 192, C::SMEM, st>>>(a);
-        BD_CHECK_LAUNCH("k_conv_wgrad");
-    }
+    k_conv_wgrad<COUT, CIS><<<dim3(grid, slices), 192, C::SMEM, st>>>(a);
+    BD_CHECK_LAUNCH("k_conv_wgrad");
     return BD_OK;
 }
 
@@ -741,11 +757,13 @@ int conv_launch(const BdConvCall& c, cudaStream_t st, int* err) {
 int wgrad_launch(int nx, int ny, int nz, int cin, int cout, int taps, const void* grad, const void* act, float* dw,
                  cudaStream_t st, int* err) {
     const int sms = sm_count();
-#define BD_WG_CASE(CO, CI) \
-    if (cout == CO && cin == CI) return launch_wgrad_t<CO, CI>(nx, ny, nz, taps, grad, act, dw, st, err, sms);
-    BD_WG_CASE(16, 16) BD_WG_CASE(16, 32) BD_WG_CASE(16, 64)
-    BD_WG_CASE(32, 16) BD_WG_CASE(32, 32) BD_WG_CASE(32, 64)
-    BD_WG_CASE(64, 16) BD_WG_CASE(64, 32) BD_WG_CASE(64, 64)
+#define BD_WG_CASE(CO, CIS_)                                                  \
+    if (cout == CO && (cin == CIS_ || (cin > CIS_ && CIS_ == 32)))            \
+        return launch_wgrad_t<CO, CIS_>(nx, ny, nz, cin, taps, grad, act, dw, st, err, sms);
+    // 64 input channels run as two slices of 32: their accumulators would not fit TMEM
+    BD_WG_CASE(16, 16) BD_WG_CASE(16, 32)
+    BD_WG_CASE(32, 16) BD_WG_CASE(32, 32)
+    BD_WG_CASE(64, 16) BD_WG_CASE(64, 32)
 #undef BD_WG_CASE
     return fail(BD_ERR_INVALID_ARG, "bd_conv3d_wgrad: unsupported channel combination");
 }

@@ -1,0 +1,32 @@
+"""Weight-gradient kernel at the edges of its row chunks, stages, splits and channel slices.
+
+Gradients and activations are whole numbers in [-3, 3], so every product and every partial sum is a
+whole number far below 2**24 (at most 9 x 16,000 voxels): FP32 accumulation is exact in any order and
+the kernel has to give the oracle's weights exactly, on top of what the buffer held before."""
+import numpy as np
+import pytest
+
+from oracle import unet as ou
+
+pytestmark = pytest.mark.gpu
+
+# one voxel; rows shorter than a core matrix; interiors of one chunk to within a row; several CTAs with a
+# ragged last range (2048 rows each); long z rows
+SHAPES = [(1, 1, 1), (3, 2, 5), (1, 7, 126), (9, 5, 14), (11, 13, 17), (20, 25, 32)]
+COMBOS = [(16, 16), (16, 32), (32, 16), (32, 32), (32, 64), (64, 16), (64, 32), (64, 64), (16, 64)]
+
+
+@pytest.mark.parametrize("taps", [27, 9])
+@pytest.mark.parametrize("cout,cin", COMBOS)
+def test_weight_gradient_is_exact_on_whole_numbers(gpu, cout, cin, taps):
+    import torch
+    from bug_defense_b200 import denoise
+    rng = np.random.default_rng(1000 * cout + 10 * cin + taps)
+    for shape in SHAPES:
+        g = rng.integers(-3, 4, size=(cout,) + shape).astype(np.float64)
+        x = rng.integers(-3, 4, size=(cin,) + shape).astype(np.float64)
+        was = rng.integers(-3, 4, size=(taps, cout, cin)).astype(np.float64)
+        dw = torch.from_numpy(was).to("cuda", torch.float32)
+        planes = [denoise.to_planes(torch.from_numpy(a).to("cuda", torch.float32)) for a in (g, x)]
+        denoise.conv3d_wgrad(planes[0], planes[1], dw, shape, cin, cout, taps=taps)
+        np.testing.assert_array_equal(dw.double().cpu().numpy(), was + ou.conv_wgrad(g, x, taps), err_msg=str(shape))
