@@ -6,18 +6,22 @@
 // 27 row-shifted GEMMs [128 voxels x cin] x [cin x cout] accumulated in TMEM (implicit GEMM), and
 // every operand tile is a run of contiguous 16-byte rows: one bulk copy per 8 channels.
 //
-// Forward / data-gradient kernel (k_conv): persistent CTAs walk tiles of 128 consecutive rows. For
-// each of the 9 (dx, dy) pairs, cin/8 bulk copies bring the tile's rows shifted by (dx, dy) into
-// shared memory, which is exactly the K-major, no-swizzle UMMA layout. The three z taps are stacked
-// along N: one 128 x (3*cout) x 16 MMA per K step accumulates D[u][(dz, co)], and the epilogue
-// forms out[v] = D[v-1][dz=-1] + D[v][dz=0] + D[v+1][dz=+1] with warp shuffles (shared memory
-// across warp edges), so a tile yields 126 outputs (rows 1..126). A pipeline stage holds 9, 3 or 1
-// of a tile's runs (as shared memory allows), so the single MMA-issuing thread waits on one barrier
-// per stage, not per run; few, wide MMAs keep the tensor pipe's issue rate off the critical path
-// for the 16-channel layers. Weights of all taps stay resident in shared memory. Warp 0 issues the
-// copies, warp 1 owns TMEM and issues tcgen05.mma, warps 2-9 (two groups, one per accumulator)
-// drain the double-buffered accumulators and run the fused epilogue (bias, ReLU, nearest
-// upsampling with the skip add, gradient gating, the 1x1 head).
+// Forward / data-gradient kernel (k_conv): a CTA computes 16 output channels of units of up to 3 tiles of 128
+// rows of the (y, z) plane, marching along x. A plane's rows arrive once, with their dy and dz halo, as cin/8
+// bulk copies: K-major, no-swizzle UMMA operands, whose (dy, dz) shift is a shift of the start address by
+// whole 16-byte rows. The plane x adds to the outputs of x-1, x and x+1 at once: the three are neighbours in
+// TMEM and stacked along N, one 128 x 48 x 16 MMA per (dy, dz) and K step, and the weights lie in shared
+// memory so that every rotation of the three slots is a run. Each z tap has accumulators of its own, summed
+// as (t0 + t-1) + t+1 at the end, which keeps the sums' order of 27 taps as (dx, dy) runs. A finished output
+// plane's slot is read, cleared for the plane three on, and goes through the fused epilogue (bias, ReLU,
+// nearest upsampling with the skip add, gradient gating, the 1x1 head), a group of 4 warps per tile. Three
+// warps issue MMAs, one a tile: the tensor pipe queues only a few, and a warp that waits for its barrier
+// leaves it idle for hundreds of clocks.
+// Bounds: an MMA of this shape takes 43 clocks whatever N <= 48 (the A rows' read), 9 per 128 rows and 16
+// channels. Reading nine shifted copies of every row instead, with N = 48 from the z taps and the z sums by
+// shuffles, was bound by the copies (36 KB and 18 copies a tile) and then by the shuffles. 16 -> 16 channels
+// at 200x200x128: 237 us before, 105 us now, of which 63 MMAs; 32 -> 16: 176 and 120; the whole network's
+// forward pass 1.31 ms and 0.86 ms, of a 100x60x64 volume 0.24 and 0.22 ms.
 //
 // Weight-gradient kernel (k_conv_wgrad): dW[(dx, dy), dz][co][ci] = sum_u g[u - (dx, dy)][co] x[u + dz][ci].
 // The nine (dx, dy)-shifted gradient tiles are stacked along M (128/cout pairs per MMA) and the three
@@ -47,11 +51,14 @@ namespace bd {
 namespace {
 
 constexpr int kTileM = 128;
-constexpr int kPlaneBytes = kTileM * 16;   // one 8-channel plane of a tile: 128 rows x 16 B
 constexpr int kSmemLimit = 232448;     // 227 KB opt-in dynamic shared memory per CTA
 constexpr int kRowMargin = 256;        // zero rows after the padded volume (tile copies overrun it)
-constexpr int kEpiGroups = 2;          // epilogue warp groups (4 warps each), one per accumulator
-constexpr int kConvThreads = 64 + kEpiGroups * 128;
+constexpr int kSlice = 16;             // output channels of a k_conv CTA
+constexpr int kMaxTiles = 3;           // tiles of a unit: 3 z taps x 3 planes x 16 TMEM columns each
+constexpr int kTileCols = 9 * kSlice;
+constexpr int kMmaWarps = kMaxTiles;
+constexpr int kEpiGroups = kMaxTiles;  // epilogue groups of 4 warps, one a tile
+constexpr int kConvThreads = (1 + kMmaWarps + 4 * kEpiGroups) * 32;
 
 struct Geom {
     int nxp, nyp, nzp;
@@ -72,13 +79,22 @@ __host__ __device__ inline Geom make_geom(int nx, int ny, int nz) {
 
 __device__ __forceinline__ size_t prow(const Geom& g, int chunk, int v) { return ((size_t)chunk * g.R + v) * 8; }
 
+// How k_conv cuts a level into units: `groups` in-plane groups of `tiles` x 128 rows, times segments of
+// `steps` planes along x.
+struct MarchPlan {
+    int tiles, groups, steps, units;
+    int segs;          // copies per plane and 8 channels: one window of rows, or the rows of dy = -1, 0, +1
+    int dy_rows;       // rows between the dy = -1, 0, +1 operands of a slot
+    int rows;          // rows of a slot
+    int slots;         // planes in shared memory
+};
+
 struct ConvArgs {
     Geom g;        // level of the convolution
     Geom gf;       // finer level (UPADD modes)
-    int taps, mode, cout_total, n_off, n_tiles;
+    int taps, mode, n_off, n_slice;
     const __nv_bfloat16* input;
     const __nv_bfloat16* wimage;
-    int wbytes;
     const float* bias;
     __nv_bfloat16* out;
     __nv_bfloat16* out_coarse;
@@ -94,6 +110,7 @@ struct ConvArgs {
     double* loss;
     __nv_bfloat16* grad_out;
     int* err;
+    MarchPlan m;
 };
 
 __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
@@ -115,24 +132,25 @@ __device__ __forceinline__ void store_row(__nv_bfloat16* base, const Geom& g, in
     }
 }
 
+__device__ __forceinline__ void unpack8(const uint4& q, float* val) {
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float2 f = __bfloat1622float2(h[j]);
+        val[2 * j] = f.x;
+        val[2 * j + 1] = f.y;
+    }
+}
+
 template <int N>
 __device__ __forceinline__ void load_row(const __nv_bfloat16* base, const Geom& g, int c0, int v, float* val) {
 #pragma unroll
-    for (int c = 0; c < N; c += 8) {
-        const uint4 q = *reinterpret_cast<const uint4*>(base + prow(g, c0 + c / 8, v));
-        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float2 f = __bfloat1622float2(h[j]);
-            val[c + 2 * j] = f.x;
-            val[c + 2 * j + 1] = f.y;
-        }
-    }
+    for (int c = 0; c < N; c += 8) unpack8(*reinterpret_cast<const uint4*>(base + prow(g, c0 + c / 8, v)), val + c);
 }
 
 struct SharedCtl {
     unsigned long long full[32], empty[32];
-    unsigned long long wfull, acc_full[2], acc_empty[2], done;
+    unsigned long long acc_full[kEpiGroups], acc_empty[kMaxTiles], done;
     uint32_t tmem;
     volatile int abort;
 };
@@ -142,6 +160,13 @@ __device__ __forceinline__ bool wait_or_abort(unsigned long long* bar, unsigned 
     ctl->abort = 1;
     if (err) atomicExch(err, 1);
     return false;
+}
+
+// The same for a whole warp, which stays converged; false also once another role has given up.
+__device__ __forceinline__ bool warp_wait(unsigned long long* bar, unsigned parity, SharedCtl* ctl, int* err) {
+    bool ok = mbar_wait_limit(bar, parity, 1);
+    if (!ok) ok = !ctl->abort && wait_or_abort(bar, parity, ctl, err);
+    return __all_sync(0xffffffffu, ok);
 }
 
 // A producer warp whose lanes all issue copies, before it fills a stage of `bytes`: false (in every lane)
@@ -158,73 +183,18 @@ __device__ __forceinline__ bool open_stage(unsigned long long* empty, unsigned p
 
 constexpr int pow2_at_least(int x) { return x <= 32 ? 32 : x <= 64 ? 64 : x <= 128 ? 128 : x <= 256 ? 256 : 512; }
 
-template <int CIN, int N>
-struct ConvCfg {
-    static constexpr int KP = CIN / 8;
-    static constexpr int RUN = KP * kPlaneBytes;   // one (dx, dy)-shifted run of a tile
-    static constexpr int WMAX = 27 * CIN * N * 2;
-    static constexpr int XB = 2 * 2 * 2 * 4 * N;  // floats: edge exchange [group][parity][side][quad][N]
-    static constexpr int CTL = 1024 + ((XB * 4 + 256 + 1023) / 1024) * 1024;  // SharedCtl + exchange + bias
-    static constexpr int AVAIL = kSmemLimit - 1024 - CTL - WMAX;
-    // runs per pipeline stage: as many of the 9 as keep >= 3 stages, so the single MMA-issuing
-    // thread waits on few barriers per tile
-    static constexpr int RPS = AVAIL / (9 * RUN) >= 3 ? 9 : AVAIL / (3 * RUN) >= 3 ? 3 : 1;
-    static constexpr int STAGE = RPS * RUN;
-    static constexpr int NST_FIT = AVAIL / STAGE;
-    static constexpr int NST = NST_FIT > 32 ? 32 : NST_FIT;
-    static constexpr int SMEM = 1024 + CTL + WMAX + NST * STAGE;
-    static constexpr int TMEM_COLS = pow2_at_least(2 * 3 * N);   // two accumulators of 3N columns
-    static_assert(NST >= 3, "conv: not enough shared memory for a 3-stage pipeline");
-    static_assert(SMEM <= kSmemLimit, "conv: shared memory over the limit");
-};
-
-// Fused epilogue for the voxel in row v of the level; acc holds its N accumulator values.
-template <int N>
-__device__ __forceinline__ void conv_epilogue(const ConvArgs& a, int v, float* acc, float* head_acc, double& loss_acc) {
+// Fused epilogue for voxel (x, y, z) of the padded level, row v; acc holds its N outputs from 8-channel plane
+// c0 on.
+template <int N, bool HEAD>
+__device__ __forceinline__ void conv_epilogue(const ConvArgs& a, int c0, int x, int y, int z, int v, float* acc,
+                                              float* head_acc, double& loss_acc) {
     const Geom& g = a.g;
-    const int x = v / g.plane, r = v - x * g.plane, y = r / g.nzp, z = r - y * g.nzp;
-    if (v >= g.v_hi || y < 1 || y > g.nyp - 2 || z < 1 || z > g.nzp - 2) return;
-    const int mode = a.mode;
+    const int mode = HEAD ? BD_CONV_FWD_HEAD : a.mode;
     if (mode <= BD_CONV_FWD_HEAD) {
 #pragma unroll
         for (int c = 0; c < N; ++c) acc[c] = fmaxf(acc[c], 0.f);
     }
-    const int c0 = a.n_off / 8;
-    if (mode == BD_CONV_FWD_RELU || mode == BD_CONV_BWD_RAW) {
-        store_row<N>(a.out, g, c0, v, acc);
-    } else if (mode == BD_CONV_BWD_MASK) {
-#pragma unroll
-        for (int c = 0; c < N; c += 8) {
-            float m[8];
-            load_row<8>(a.aux, g, c0 + c / 8, v, m);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) acc[c + j] = m[j] > 0.f ? acc[c + j] : 0.f;
-        }
-        store_row<N>(a.out, g, c0, v, acc);
-    } else if (mode == BD_CONV_FWD_UPADD || mode == BD_CONV_BWD_UPADD) {
-        if (mode == BD_CONV_FWD_UPADD && a.out_coarse) store_row<N>(a.out_coarse, g, c0, v, acc);
-        const Geom& f = a.gf;
-        for (int ch = 0; ch < 8; ++ch) {
-            const int fx = 2 * x - 1 + (ch >> 2), fy = 2 * y - 1 + ((ch >> 1) & 1), fz = 2 * z - 1 + (ch & 1);
-            const int vf = fx * f.plane + fy * f.nzp + fz;
-#pragma unroll
-            for (int c = 0; c < N; c += 8) {
-                float s[8], o[8];
-                load_row<8>(a.aux, f, c0 + c / 8, vf, s);
-                if (mode == BD_CONV_FWD_UPADD) {
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) o[j] = acc[c + j] + s[j];
-                } else {
-                    float m[8];
-                    load_row<8>(a.aux2, f, c0 + c / 8, vf, m);
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) o[j] = m[j] > 0.f ? s[j] + 0.125f * acc[c + j] : 0.f;
-                }
-                store_row<8>(a.out, f, c0 + c / 8, vf, o);
-            }
-        }
-    } else if constexpr (N == 16) {
-        if (mode != BD_CONV_FWD_HEAD) return;
+    if constexpr (HEAD) {
         const int nz = g.nzp - 2, ny = g.nyp - 2;
         const size_t u = ((size_t)(x - 1) * ny + (y - 1)) * nz + (z - 1);
         float yv = a.head[N];
@@ -246,221 +216,321 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs& a, int v, float* a
             head_acc[N] += dy;
             store_row<N>(a.grad_out, g, 0, v, gr);
         }
+        return;
+    }
+    if (mode == BD_CONV_FWD_RELU || mode == BD_CONV_BWD_RAW) {
+        store_row<N>(a.out, g, c0, v, acc);
+    } else if (mode == BD_CONV_BWD_MASK) {
+#pragma unroll
+        for (int c = 0; c < N; c += 8) {
+            float m[8];
+            load_row<8>(a.aux, g, c0 + c / 8, v, m);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[c + j] = m[j] > 0.f ? acc[c + j] : 0.f;
+        }
+        store_row<N>(a.out, g, c0, v, acc);
+    } else if (mode == BD_CONV_FWD_UPADD || mode == BD_CONV_BWD_UPADD) {
+        if (mode == BD_CONV_FWD_UPADD && a.out_coarse) store_row<N>(a.out_coarse, g, c0, v, acc);
+        const Geom& f = a.gf;
+        // the eight fine voxels of 8 channels at a time, all loads before the first store
+        const int vf0 = (2 * x - 1) * f.plane + (2 * y - 1) * f.nzp + 2 * z - 1;
+#pragma unroll
+        for (int c = 0; c < N; c += 8) {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                uint4 s[4], m[4];
+                int vf[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    vf[k] = vf0 + h * f.plane + (k >> 1) * f.nzp + (k & 1);
+                    s[k] = *reinterpret_cast<const uint4*>(a.aux + prow(f, c0 + c / 8, vf[k]));
+                    if (mode == BD_CONV_BWD_UPADD)
+                        m[k] = *reinterpret_cast<const uint4*>(a.aux2 + prow(f, c0 + c / 8, vf[k]));
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    float sv[8], mv[8], o[8];
+                    unpack8(s[k], sv);
+                    if (mode == BD_CONV_FWD_UPADD) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) o[j] = acc[c + j] + sv[j];
+                    } else {
+                        unpack8(m[k], mv);
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) o[j] = mv[j] > 0.f ? sv[j] + 0.125f * acc[c + j] : 0.f;
+                    }
+                    store_row<8>(a.out, f, c0 + c / 8, vf[k], o);
+                }
+            }
+        }
     }
 }
 
-template <int CIN, int N>
+// A warp's share of the head's weight gradient and of the loss.
+template <int HA>
+__device__ __forceinline__ void flush_head(const ConvArgs& a, const float* head_acc, double loss_acc, int lane) {
+    if (!a.target) return;
+#pragma unroll
+    for (int c = 0; c < HA; ++c) {
+        float h = head_acc[c];
+        for (int o = 16; o; o >>= 1) h += __shfl_xor_sync(0xffffffffu, h, o);
+        if (lane == 0) atomicAdd(&a.head_grad[c], h);
+    }
+    for (int o = 16; o; o >>= 1) loss_acc += __shfl_xor_sync(0xffffffffu, loss_acc, o);
+    if (lane == 0) atomicAdd(a.loss, loss_acc);
+}
+
+template <int CIN>
+struct ConvCfg {
+    static constexpr int KP = CIN / 8;
+    static constexpr int WBLK = kSlice * 16;       // 16 outputs x 8 input channels of one tap
+    static constexpr int WK = 5 * WBLK;            // dx = +1, 0, -1, +1, 0: every rotation is a run of three
+    static constexpr int WMAX = 9 * KP * WK;
+    static constexpr int CTL = 1024;               // SharedCtl + bias
+    static constexpr int AVAIL = kSmemLimit - 1024 - CTL - WMAX;   // for the planes
+};
+
+// Slice blockIdx.y of 16 outputs. See the file comment for the layout and march_plan for the units.
+template <int CIN, bool HEAD>
 __global__ void __launch_bounds__(kConvThreads, 1) k_conv(const ConvArgs a) {
-    using C = ConvCfg<CIN, N>;
+    using C = ConvCfg<CIN>;
     extern __shared__ unsigned char smem_raw[];
     const uint32_t base_addr = smem_addr(smem_raw);
     unsigned char* smem = smem_raw + ((1024 - (base_addr & 1023)) & 1023);
     SharedCtl* ctl = reinterpret_cast<SharedCtl*>(smem);
+    float* sbias = reinterpret_cast<float*>(smem + C::CTL - kSlice * 4);   // bias (forward modes), else 0
     unsigned char* wsm = smem + C::CTL;
-    unsigned char* stages = wsm + C::WMAX;
-
-    float* xbuf = reinterpret_cast<float*>(smem + 1024);
-    float* sbias = xbuf + C::XB;                    // [N] bias of the slice (forward modes), else 0
+    unsigned char* planes = wsm + C::WMAX;
+    static_assert(sizeof(SharedCtl) + kSlice * 4 <= C::CTL, "conv: control block over its space");
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int kz = a.taps == 27 ? 3 : 1;
-    const int NN = kz * N;                          // MMA N: z taps stacked along N
-    const int out_per_tile = kz == 3 ? kTileM - 2 : kTileM;
-    const int u_base = a.g.v_lo - (kz == 3 ? 1 : 0);
+    const MarchPlan m = a.m;
+    const int nx = a.g.nxp - 2, group_rows = m.tiles * kTileM;
+    const int in_rows = (a.g.nyp - 2) * a.g.nzp - 2;   // in-plane rows from the first interior one to the last
+    const uint32_t kp_bytes = m.rows * 16, slot_bytes = C::KP * kp_bytes;
+    const int n0 = blockIdx.y * kSlice;
+    const int issuers = m.tiles == 1 ? kz : m.tiles;           // MMA warps at work: one a z tap, or one a tile
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < C::NST; ++s) {
+        for (int s = 0; s < m.slots; ++s) {
             mbar_init(&ctl->full[s], 1);
-            mbar_init(&ctl->empty[s], 1);
+            mbar_init(&ctl->empty[s], issuers);
         }
-        mbar_init(&ctl->wfull, 1);
-        for (int i = 0; i < 2; ++i) {
-            mbar_init(&ctl->acc_full[i], 1);
-            mbar_init(&ctl->acc_empty[i], 128);
-        }
-        mbar_init(&ctl->done, 1);
+        for (int i = 0; i < kEpiGroups; ++i) mbar_init(&ctl->acc_full[i], m.tiles == 1 ? kz : 1);
+        for (int i = 0; i < kMaxTiles; ++i) mbar_init(&ctl->acc_empty[i], 4);
+        mbar_init(&ctl->done, issuers);
         ctl->abort = 0;
         mbar_init_fence();
     }
-    for (int c = threadIdx.x; c < N; c += blockDim.x)
-        sbias[c] = (a.mode <= BD_CONV_FWD_HEAD && a.bias) ? a.bias[c] : 0.f;
-    if (warp == 1) tmem_alloc(&ctl->tmem, C::TMEM_COLS);
+    if (threadIdx.x < kSlice)
+        sbias[threadIdx.x] = (a.mode <= BD_CONV_FWD_HEAD && a.bias) ? a.bias[n0 + threadIdx.x] : 0.f;
+    if (warp == 1) tmem_alloc(&ctl->tmem, 512);
+    // resident weights, wsm[dy][dz][k plane][5 dx][16 outputs][8], by plain loads: a bulk copy takes ~100
+    // clocks to issue whatever its size, and these would be 256-byte ones
+    for (int i = threadIdx.x; i < 3 * kz * C::KP * 5 * kSlice; i += kConvThreads) {
+        const int n = i % kSlice, blk = i / kSlice % 5, r = i / kSlice / 5, kp = r % C::KP, t = r / C::KP;
+        const int dz = t % kz, dy = t / kz, dx = 2 - blk % 3;       // 2, 1, 0 = +1, 0, -1
+        reinterpret_cast<uint4*>(wsm)[i] = *reinterpret_cast<const uint4*>(
+            a.wimage + ((((dx * 3 + dy) * C::KP + kp) * kz + dz) * a.n_slice + n0 + n) * 8);
+    }
+    fence_proxy_async_smem();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = ctl->tmem;
+    const uint32_t tmem = uniform(ctl->tmem);
+    const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;      // TMEM lanes of an epilogue warp
+    if (warp >= 4 && warp < 8) {
+        for (int c = 0; c < kMaxTiles * kTileCols; c += 16) tmem_zero16(tmem + lanes + c);
+        tmem_st_wait();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
 
     if (warp == 0) {
+        // ---- producer: the units' planes x0-1 .. x1+1 one after another ----
         if (lane == 0) {
-            // ---- producer: resident weights, then 9 (dx, dy)-shifted row runs per tile ----
-            mbar_expect_tx(&ctl->wfull, a.wbytes);
-            for (int off = 0; off < a.wbytes; off += 32768)
-                bulk_load(wsm + off, reinterpret_cast<const unsigned char*>(a.wimage) + off,
-                          min(32768, a.wbytes - off), &ctl->wfull);
             int s = 0;
             unsigned ph = 0;
             long long issued = 0;
-            for (int tile = blockIdx.x; tile < a.n_tiles && !ctl->abort; tile += gridDim.x) {
-                const int u0 = u_base + tile * out_per_tile;
-                for (int q0 = 0; q0 < 9; q0 += C::RPS) {
-                    if (!wait_or_abort(&ctl->empty[s], ph ^ 1, ctl, a.err)) break;
-                    unsigned char* st = stages + s * C::STAGE;
-                    mbar_expect_tx(&ctl->full[s], C::STAGE);
+            bool ok = true;
+            const int seg_rows = m.segs == 1 ? m.rows : m.dy_rows;
+            for (int unit = blockIdx.x; ok && unit < m.units; unit += gridDim.x) {
+                const int x0 = 1 + unit / m.groups * m.steps, x1 = min(nx, x0 + m.steps - 1);
+                const int p = unit % m.groups * group_rows;    // (dy, dz) = (-1, -1) row of the first output
+                for (int x = x0 - 1; x <= x1 + 1; ++x) {
+                    ok = !ctl->abort && wait_or_abort(&ctl->empty[s], ph ^ 1, ctl, a.err);
+                    if (!ok) break;
+                    const int row0 = x * a.g.plane + p;
+                    // a group that overruns the last plane stops at the volume's end
+                    uint32_t bytes = 0;
+                    for (int i = 0; i < m.segs; ++i) bytes += min(seg_rows, a.g.R - (row0 + i * a.g.nzp)) * 16;
+                    mbar_expect_tx(&ctl->full[s], C::KP * bytes);
+                    for (int i = 0; i < m.segs; ++i) {
+                        const int row = row0 + i * a.g.nzp;
+                        const uint32_t n = min(seg_rows, a.g.R - row) * 16;
 #pragma unroll
-                    for (int r = 0; r < C::RPS; ++r) {
-                        const int q = q0 + r;
-                        const int row0 = u0 + (q / 3 - 1) * a.g.plane + (q % 3 - 1) * a.g.nzp;
-#pragma unroll
-                        for (int p = 0; p < C::KP; ++p)
-                            bulk_load(st + r * C::RUN + p * kPlaneBytes, a.input + prow(a.g, p, row0), kPlaneBytes,
-                                      &ctl->full[s]);
+                        for (int k = 0; k < C::KP; ++k)
+                            bulk_load(planes + s * slot_bytes + k * kp_bytes + i * m.dy_rows * 16,
+                                      a.input + prow(a.g, k, row), n, &ctl->full[s]);
                     }
                     ++issued;
-                    if (++s == C::NST) { s = 0; ph ^= 1; }
+                    if (++s == m.slots) { s = 0; ph ^= 1; }
                 }
             }
             // drain: every issued load has landed before the CTA leaves
-            const long long n_drain = issued < C::NST ? issued : C::NST;
+            const long long n_drain = issued < m.slots ? issued : m.slots;
             for (long long i = 0; i < n_drain; ++i) {
-                if (--s < 0) { s = C::NST - 1; ph ^= 1; }
+                if (--s < 0) { s = m.slots - 1; ph ^= 1; }
                 mbar_wait(&ctl->full[s], ph);
             }
-            mbar_wait(&ctl->wfull, 0);
         }
-    } else if (warp == 1) {
-        if (lane == 0) {
-            // ---- MMA issuer: per (dx, dy) stage, CIN/16 MMAs of 128 x NN x 16 ----
-            const uint32_t idesc = umma_idesc_bf16(kTileM, NN, false, false);
-            const uint32_t wbase = smem_addr(wsm), sbase = smem_addr(stages);
-            const uint32_t wq = C::KP * NN * 16;    // weight image bytes per (dx, dy) pair
-            bool ok = wait_or_abort(&ctl->wfull, 0, ctl, a.err);
-            int s = 0, acc = 0;
-            unsigned ph = 0, aph = 0;
-            for (int tile = blockIdx.x; ok && tile < a.n_tiles && !ctl->abort; tile += gridDim.x) {
-                if (!wait_or_abort(&ctl->acc_empty[acc], aph ^ 1, ctl, a.err)) break;
-                tc_fence_after();
-                const uint32_t d = tmem + acc * NN;
-                for (int q0 = 0; q0 < 9 && ok; q0 += C::RPS) {
-                    if (!wait_or_abort(&ctl->full[s], ph, ctl, a.err)) { ok = false; break; }
+        __syncwarp();
+    } else if (warp <= kMmaWarps) {
+        // ---- MMA issuers: per plane and tile 3 * kz * CIN/16 MMAs of 128 x 48 x 16. Every tile's (or z tap's)
+        // MMAs come from one warp, in order ----
+        const int me = uniform(warp - 1);
+        const int my_t = m.tiles == 1 ? 0 : me, dz0 = m.tiles == 1 ? me : 0, dz1 = m.tiles == 1 ? me + 1 : kz;
+        const uint32_t lead = elect_one();
+        constexpr uint32_t idesc48 = umma_idesc_bf16(kTileM, 3 * kSlice, false, false);
+        constexpr uint32_t idesc16 = umma_idesc_bf16(kTileM, kSlice, false, false);
+        const uint32_t wbase = smem_addr(wsm), pbase = smem_addr(planes);
+        bool ok = me < issuers;
+        int s = 0, turn = my_t, oldest = 0;
+        unsigned ph = 0, eph = 0;
+        bool drained = false;
+        for (int unit = blockIdx.x; ok && unit < m.units; unit += gridDim.x) {
+            const int x0 = 1 + unit / m.groups * m.steps;
+            const int planes_n = uniform(min(nx + 1 - x0, m.steps) + 2);
+            const int left = in_rows - unit % m.groups * group_rows;
+            const int tiles = uniform(min(m.tiles, (left + kTileM - 1) / kTileM));
+            for (int i = 0; i < planes_n; ++i) {                    // plane x = x0 - 1 + i
+                ok = warp_wait(&ctl->full[s], ph, ctl, a.err);
+                if (!ok) break;
+                if (my_t < tiles) {
+                    if (drained) {       // slot x+1 is the one that the plane before this completed
+                        ok = warp_wait(&ctl->acc_empty[my_t], eph, ctl, a.err);
+                        if (!ok) break;
+                        eph ^= 1;
+                    }
                     tc_fence_after();
-                    const uint32_t st = sbase + s * C::STAGE;
+                    // outputs x-1, x, x+1 live in slots oldest, oldest+1, oldest+2 (mod 3); a unit's first two
+                    // and last two planes add to its own outputs only
+                    const uint32_t wrot = wbase + (oldest ? 3 - oldest : 0) * C::WBLK;
+                    const uint32_t op = pbase + s * slot_bytes + my_t * kTileM * 16 + (kz == 3 ? 0 : 16);
+                    const uint32_t d = tmem + my_t * kTileCols;
+                    const uint32_t mine = (i >= 2) | (i >= 1 && i < planes_n - 1) << 1 | (i < planes_n - 2) << 2;
+                    const int pieces = mine == 7 ? 1 : 3;
+                    for (int k = 0; k < pieces; ++k) {
+                        if (!(mine >> k & 1)) continue;
+                        const int at = mine == 7 ? 0 : oldest + k - (oldest + k >= 3 ? 3 : 0);   // slot of x - 1 + k
+                        const uint32_t idesc = mine == 7 ? idesc48 : idesc16;
+                        for (int dz = dz0; dz < dz1; ++dz) {
 #pragma unroll
-                    for (int r = 0; r < C::RPS; ++r) {
-                        const int q = q0 + r;
+                            for (int dy = 0; dy < 3; ++dy)
 #pragma unroll
-                        for (int kk = 0; kk < CIN / 16; ++kk) {
-                            const uint64_t ad = umma_desc(st + r * C::RUN + kk * 2 * kPlaneBytes, kPlaneBytes, 128,
-                                                          UMMA_NONE);
-                            const uint64_t bd = umma_desc(wbase + q * wq + kk * 2 * (NN * 16), NN * 16, 128, UMMA_NONE);
-                            umma_bf16(d, ad, bd, idesc, (q | kk) != 0);
+                                for (int kk = 0; kk < CIN / 16; ++kk) {
+                                    const uint64_t ad = umma_desc(op + (dy * m.dy_rows + dz) * 16 + kk * 2 * kp_bytes,
+                                                                  kp_bytes, 128, UMMA_NONE);
+                                    const uint64_t bd = umma_desc(
+                                        wrot + ((dy * kz + dz) * C::KP + kk * 2) * C::WK + at * C::WBLK, C::WK, 128, UMMA_NONE);
+                                    umma_bf16(d + (dz * 3 + at) * kSlice, ad, bd, idesc, true, lead);
+                                }
                         }
                     }
-                    umma_commit(&ctl->empty[s]);
-                    if (++s == C::NST) { s = 0; ph ^= 1; }
+                    drained = i >= 2;
+                    if (drained) {
+                        umma_commit(&ctl->acc_full[turn], lead);
+                        if (m.tiles == 1 && ++turn == kEpiGroups) turn = 0;
+                    }
                 }
-                if (!ok) break;
-                umma_commit(&ctl->acc_full[acc]);
-                acc ^= 1;
-                if (acc == 0) aph ^= 1;
+                umma_commit(&ctl->empty[s], lead);
+                if (++s == m.slots) { s = 0; ph ^= 1; }
+                if (++oldest == 3) oldest = 0;
             }
-            umma_commit(&ctl->done);
+        }
+        if (me < issuers) {
+            umma_commit(&ctl->done, lead);
             mbar_wait(&ctl->done, 0);
         }
+        __syncwarp();
     } else {
-        // ---- epilogue: two groups of 4 warps (2..5, 6..9); group g drains accumulator g, i.e.
-        // every other tile of this CTA. Warp w reads TMEM lanes 32*(w % 4) .. +31; row = TMEM lane.
-        const int grp = (warp - 2) >> 2;
-        const int quad = warp & 3;
-        const int row = quad * 32 + lane;
-        const int acc = grp;
-        unsigned aph = 0;
-        constexpr int HA = N == 16 ? 17 : 1;        // head gradient accumulators (16-channel head only)
-        float head_acc[HA];
-#pragma unroll
-        for (int c = 0; c < HA; ++c) head_acc[c] = 0.f;
+        // ---- epilogue: a group of 4 warps for each tile; one tile a unit goes round the groups. Warp w
+        // reads TMEM lanes 32*(w % 4) .. +31; row = TMEM lane. ----
+        const int grp = (warp - 1 - kMmaWarps) >> 2;
+        const int t = m.tiles == 1 ? 0 : grp;
+        const int row = (warp & 3) * 32 + lane;
+        const int c0 = (a.n_off + n0) / 8;
+        unsigned ph = 0;
+        float head_acc[HEAD ? kSlice + 1 : 1];
         double loss_acc = 0.0;
-        int par = 0;
-        for (int tile = blockIdx.x + grp * gridDim.x; tile < a.n_tiles; tile += kEpiGroups * gridDim.x) {
-            // a timed-out wait still takes part in the group's named barrier below, so its four
-            // warps stay in step; the tile is then skipped
-            const bool okw = !ctl->abort && wait_or_abort(&ctl->acc_full[acc], aph, ctl, a.err);
-            float v[N];
-            float* xb0 = xbuf + (((grp * 2 + par) * 2 + 0) * 4) * N;   // lane 31's dz=-1 block, per quad
-            float* xb2 = xbuf + (((grp * 2 + par) * 2 + 1) * 4) * N;   // lane 0's dz=+1 block, per quad
-            if (okw) {
-                tc_fence_after();
-                const uint32_t tb = tmem + ((uint32_t)(quad * 32) << 16) + acc * NN;
-                if (kz == 3) {
+        if constexpr (HEAD) {
 #pragma unroll
-                    for (int c = 0; c < N; c += 16) {
-                        float t0[16], t1[16], t2[16];
-                        tmem_ld16(tb + c, t0);
-                        tmem_ld16(tb + N + c, t1);
-                        tmem_ld16(tb + 2 * N + c, t2);
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) {
-                            const float up = __shfl_up_sync(0xffffffffu, t0[j], 1);
-                            const float dn = __shfl_down_sync(0xffffffffu, t2[j], 1);
-                            v[c + j] = t1[j] + (lane > 0 ? up : 0.f) + (lane < 31 ? dn : 0.f);
-                        }
-                        if (lane == 31) {
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) xb0[quad * N + c + j] = t0[j];
-                        }
-                        if (lane == 0) {
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) xb2[quad * N + c + j] = t2[j];
-                        }
+            for (int c = 0; c <= kSlice; ++c) head_acc[c] = 0.f;
+        }
+        int turn = 0, oldest = 0;
+        bool ok = true;
+        for (int unit = blockIdx.x; ok && unit < m.units; unit += gridDim.x) {
+            const int x0 = 1 + unit / m.groups * m.steps, x1 = min(nx, x0 + m.steps - 1);
+            const int p = unit % m.groups * group_rows;
+            const bool used = t < m.tiles && t * kTileM < in_rows - p;
+            const int r = a.g.nzp + 1 + p + t * kTileM + row, y = r / a.g.nzp, z = r - y * a.g.nzp;
+            const bool inside = y <= a.g.nyp - 2 && z >= 1 && z <= a.g.nzp - 2;
+            if (++oldest == 3) oldest = 0;                       // the planes x0 - 1 and x0 complete none
+            if (++oldest == 3) oldest = 0;
+            for (int x = x0; x <= x1; ++x) {                     // plane x + 1 completes output plane x
+                const bool mine = m.tiles == 1 ? turn == grp : used;
+                if (++turn == kEpiGroups) turn = 0;
+                if (mine) {
+                    const int vr = x * a.g.plane + r;
+                    // the order of the two additions below is a function of the voxel's row
+                    const bool late = ((vr - a.g.v_lo) % 126 & 31) == 31;
+                    ok = warp_wait(&ctl->acc_full[grp], ph, ctl, a.err);
+                    if (!ok) break;
+                    ph ^= 1;
+                    tc_fence_after();
+                    const uint32_t tb = tmem + lanes + t * kTileCols + oldest * kSlice;
+                    float v[kSlice], up[kSlice], dn[kSlice];
+                    if (kz == 3) {
+                        tmem_ld16(tb, up);
+                        tmem_ld16(tb + 3 * kSlice, v);
+                        tmem_ld16(tb + 6 * kSlice, dn);
+                    } else {
+                        tmem_ld16(tb, v);
                     }
-                } else {
-#pragma unroll
-                    for (int c = 0; c < N; c += 16) tmem_ld16(tb + c, v + c);
                     tmem_ld_wait();
-                }
-                tc_fence_before();
-            }
-            mbar_arrive(&ctl->acc_empty[acc]);
-            asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
-            if (okw && kz == 3) {
-                if (lane == 0 && quad > 0) {
+                    tmem_zero16(tb);                             // output plane x + 3 adds up here from zero
+                    if (kz == 3) {
+                        tmem_zero16(tb + 3 * kSlice);
+                        tmem_zero16(tb + 6 * kSlice);
+                    }
+                    tmem_st_wait();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&ctl->acc_empty[t]);
+                    if (inside) {
+                        if (kz == 3) {
 #pragma unroll
-                    for (int c = 0; c < N; ++c) v[c] += xb0[(quad - 1) * N + c];
-                }
-                if (lane == 31 && quad < 3) {
+                            for (int c = 0; c < kSlice; ++c)
+                                v[c] = (v[c] + (late ? dn[c] : up[c])) + (late ? up[c] : dn[c]);
+                        }
 #pragma unroll
-                    for (int c = 0; c < N; ++c) v[c] += xb2[(quad + 1) * N + c];
+                        for (int c = 0; c < kSlice; ++c) v[c] += sbias[c];
+                        conv_epilogue<kSlice, HEAD>(a, c0, x, y, z, vr, v, head_acc, loss_acc);
+                    }
                 }
+                if (++oldest == 3) oldest = 0;
             }
-            const int u0 = u_base + tile * out_per_tile;
-            const bool out_row = kz == 1 || (row >= 1 && row <= kTileM - 2);
-            if (okw && out_row && !ctl->abort) {
-#pragma unroll
-                for (int c = 0; c < N; ++c) v[c] += sbias[c];
-                conv_epilogue<N>(a, u0 + row, v, head_acc, loss_acc);
-            }
-            aph ^= 1;
-            par ^= 1;
         }
-        if (a.mode == BD_CONV_FWD_HEAD && a.target) {
-#pragma unroll
-            for (int c = 0; c < HA; ++c) {
-                float h = head_acc[c];
-                for (int o = 16; o; o >>= 1) h += __shfl_xor_sync(0xffffffffu, h, o);
-                if (lane == 0) atomicAdd(&a.head_grad[c], h);
-            }
-            for (int o = 16; o; o >>= 1) loss_acc += __shfl_xor_sync(0xffffffffu, loss_acc, o);
-            if (lane == 0) atomicAdd(a.loss, loss_acc);
-        }
+        if constexpr (HEAD) flush_head<kSlice + 1>(a, head_acc, loss_acc, lane);
     }
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem, C::TMEM_COLS);
+        tmem_dealloc(tmem, 512);
     }
 }
-
-// ------------------------------------------------------------------ weight gradient
 
 struct WgradArgs {
     Geom g;
@@ -524,7 +594,7 @@ __global__ void __launch_bounds__(192, 1) k_conv_wgrad(const WgradArgs a) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = ctl->tmem;
+    const uint32_t tmem = uniform(ctl->tmem);
 
     if (warp == 0) {
         const uint32_t bytes = 9 * C::ABOX + kz * C::BBOX;
@@ -561,32 +631,32 @@ __global__ void __launch_bounds__(192, 1) k_conv_wgrad(const WgradArgs a) {
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {
-            // MN-major, no swizzle: 8 M (or N) elements x 8 K rows per 128-byte core matrix; K groups
-            // 128 B apart (LBO), 8-element M/N blocks one chunk apart (SBO)
-            const uint32_t idesc = umma_idesc_bf16(kTileM, NN, true, true);
-            const uint32_t sbase = smem_addr(stages);
-            int s = 0;
-            unsigned ph = 0;
-            for (int c = c_begin; c < c_end && !ctl->abort; ++c) {
-                if (!wait_or_abort(&ctl->full[s], ph, ctl, a.err)) break;
-                tc_fence_after();
-                const uint32_t st = sbase + s * C::STAGE;
+        // MN-major, no swizzle: 8 M (or N) elements x 8 K rows per 128-byte core matrix; K groups
+        // 128 B apart (LBO), 8-element M/N blocks one chunk apart (SBO)
+        const uint32_t lead = elect_one();
+        const uint32_t idesc = umma_idesc_bf16(kTileM, NN, true, true);
+        const uint32_t sbase = smem_addr(stages);
+        int s = 0;
+        unsigned ph = 0;
+        for (int c = c_begin; c < c_end; ++c) {
+            if (!warp_wait(&ctl->full[s], ph, ctl, a.err)) break;
+            tc_fence_after();
+            const uint32_t st = sbase + s * C::STAGE;
 #pragma unroll
-                for (int kk = 0; kk < C::KV / 16; ++kk) {
-                    const uint64_t bd = umma_desc(st + 9 * C::ABOX + kk * 256, 128, C::CHUNK, UMMA_NONE);
+            for (int kk = 0; kk < C::KV / 16; ++kk) {
+                const uint64_t bd = umma_desc(st + 9 * C::ABOX + kk * 256, 128, C::CHUNK, UMMA_NONE);
 #pragma unroll
-                    for (int gi = 0; gi < C::NG; ++gi) {
-                        const uint64_t ad = umma_desc(st + C::pair0(gi) * C::ABOX + kk * 256, 128, C::CHUNK, UMMA_NONE);
-                        umma_bf16(tmem + gi * NN, ad, bd, idesc, (c != c_begin) || kk != 0);
-                    }
+                for (int gi = 0; gi < C::NG; ++gi) {
+                    const uint64_t ad = umma_desc(st + C::pair0(gi) * C::ABOX + kk * 256, 128, C::CHUNK, UMMA_NONE);
+                    umma_bf16(tmem + gi * NN, ad, bd, idesc, (c != c_begin) || kk != 0, lead);
                 }
-                umma_commit(&ctl->empty[s]);
-                if (++s == C::NST) { s = 0; ph ^= 1; }
             }
-            umma_commit(&ctl->acc_full[0]);
-            mbar_wait(&ctl->acc_full[0], 0);
+            umma_commit(&ctl->empty[s], lead);
+            if (++s == C::NST) { s = 0; ph ^= 1; }
         }
+        umma_commit(&ctl->acc_full[0], lead);
+        mbar_wait(&ctl->acc_full[0], 0);
+        __syncwarp();
     } else if (c_begin < c_end) {
         const int quad = warp & 3;
         const int row = quad * 32 + lane;
@@ -644,19 +714,52 @@ __global__ void k_pack_weights(int taps, int cin, int cout, int n_off, int n_sli
     }
 }
 
-template <int CIN, int N>
+// Units of k_conv, by the clocks of a CTA: a tile's MMAs at ~75 clocks each with their waits, or its epilogue
+// (~650), and a plane's load at ~24 bytes a clock; fits 43 to 75 give the same times to 2%. A unit reads two planes more than it writes, and a short group its dy halo too
+// often; the units should fill the CTAs evenly.
+MarchPlan march_plan(const Geom& g, int cin, int taps, int avail, int ctas) {
+    const int nx = g.nxp - 2, in_rows = (g.nyp - 2) * g.nzp - 2;
+    const double tile_clk = std::max(650.0, 75.0 * (taps / 3) * (cin / 16));
+    MarchPlan best{};
+    double best_cost = 0;
+    for (int tiles = 1; tiles <= kMaxTiles; ++tiles) {
+        MarchPlan m{};
+        m.tiles = tiles;
+        const int run = tiles * kTileM + 2;
+        m.segs = g.nzp <= run ? 1 : 3;
+        m.dy_rows = std::min(g.nzp, run);
+        m.rows = run + 2 * m.dy_rows;
+        m.slots = std::min(4, avail / (m.rows * cin * 2));
+        if (m.slots < 2) break;
+        m.groups = (in_rows + tiles * kTileM - 1) / (tiles * kTileM);
+        for (int cut = 1; cut <= nx && (cut == 1 || m.groups * cut <= 8 * ctas); ++cut) {
+            m.steps = (nx + cut - 1) / cut;
+            m.units = m.groups * ((nx + m.steps - 1) / m.steps);
+            const int waves = (m.units + ctas - 1) / ctas;
+            // one tile at a time: the next plane's MMAs wait for its epilogue's reads
+            const double cost = waves * (m.steps + 2.0) *
+                                std::max(tiles * tile_clk + (tiles == 1 ? 500.0 : 0.0), m.rows * cin / 12.0);
+            if (best_cost == 0 || cost < best_cost) {
+                best_cost = cost;
+                best = m;
+            }
+        }
+        if (m.groups == 1) break;
+    }
+    return best;
+}
+
+template <int CIN, bool HEAD>
 int launch_conv_t(const BdConvCall& c, cudaStream_t st, int* err, int sms) {
-    using C = ConvCfg<CIN, N>;
-    const Geom g = make_geom(c.nx, c.ny, c.nz);
+    using C = ConvCfg<CIN>;
+    // one tile a unit and two planes always fit
+    static_assert(2 * 3 * (kTileM + 2) * CIN * 2 <= C::AVAIL, "conv: not enough shared memory for two planes");
     ConvArgs a{};
-    a.g = g;
+    a.g = make_geom(c.nx, c.ny, c.nz);
     a.gf = make_geom(2 * c.nx, 2 * c.ny, 2 * c.nz);
-    a.taps = c.taps; a.mode = c.mode; a.cout_total = c.cout_total; a.n_off = c.n_off;
-    const int per_tile = c.taps == 27 ? kTileM - 2 : kTileM;
-    a.n_tiles = (g.v_hi - g.v_lo + per_tile - 1) / per_tile;
+    a.taps = c.taps; a.mode = c.mode; a.n_off = c.n_off; a.n_slice = c.n_slice;
     a.input = static_cast<const __nv_bfloat16*>(c.input);
     a.wimage = static_cast<const __nv_bfloat16*>(c.wimage);
-    a.wbytes = (int)bd_conv_image_bytes(c.taps, CIN, N);
     a.bias = c.bias;
     a.out = static_cast<__nv_bfloat16*>(c.out);
     a.out_coarse = static_cast<__nv_bfloat16*>(c.out_coarse);
@@ -666,11 +769,11 @@ int launch_conv_t(const BdConvCall& c, cudaStream_t st, int* err, int sms) {
     a.pred = c.pred; a.target = c.target; a.head_grad = c.head_grad; a.loss = c.loss;
     a.grad_out = static_cast<__nv_bfloat16*>(c.grad_out);
     a.err = err;
-    BD_CUDA(cudaFuncSetAttribute(k_conv<CIN, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
-    int occ = 1;
-    BD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_conv<CIN, N>, kConvThreads, C::SMEM));
-    const int grid = std::max(1, std::min(a.n_tiles, sms * std::max(1, occ)));
-    k_conv<CIN, N><<<grid, kConvThreads, C::SMEM, st>>>(a);
+    const int slices = c.n_slice / kSlice, ctas = std::max(1, sms / slices);
+    a.m = march_plan(a.g, CIN, c.taps, C::AVAIL, ctas);
+    const int smem = 1024 + C::CTL + C::WMAX + a.m.slots * a.m.rows * CIN * 2;
+    BD_CUDA(cudaFuncSetAttribute(k_conv<CIN, HEAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
+    k_conv<CIN, HEAD><<<dim3(std::min(a.m.units, ctas), slices), kConvThreads, smem, st>>>(a);
     BD_CHECK_LAUNCH("k_conv");
     return BD_OK;
 }
@@ -745,11 +848,10 @@ int conv_check(const BdConvCall& c) {
 
 int conv_launch(const BdConvCall& c, cudaStream_t st, int* err) {
     const int sms = sm_count();
-#define BD_CONV_CASE(CI, NN) \
-    if (c.cin == CI && c.n_slice == NN) return launch_conv_t<CI, NN>(c, st, err, sms);
-    BD_CONV_CASE(16, 16) BD_CONV_CASE(16, 32) BD_CONV_CASE(16, 64)
-    BD_CONV_CASE(32, 16) BD_CONV_CASE(32, 32) BD_CONV_CASE(32, 64)
-    BD_CONV_CASE(64, 16) BD_CONV_CASE(64, 32)
+    const bool head = c.mode == BD_CONV_FWD_HEAD;
+#define BD_CONV_CASE(CI) \
+    if (c.cin == CI) return head ? launch_conv_t<CI, true>(c, st, err, sms) : launch_conv_t<CI, false>(c, st, err, sms);
+    BD_CONV_CASE(16) BD_CONV_CASE(32) BD_CONV_CASE(64)
 #undef BD_CONV_CASE
     return fail(BD_ERR_INVALID_ARG, "bd_conv3d: unsupported channel combination");
 }
