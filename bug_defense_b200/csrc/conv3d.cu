@@ -24,15 +24,16 @@
 // forward pass 1.31 ms and 0.86 ms, of a 100x60x64 volume 0.24 and 0.22 ms.
 //
 // Weight-gradient kernel (k_conv_wgrad): dW[(dx, dy), dz][co][ci] = sum_u g[u - (dx, dy)][co] x[u + dz][ci].
-// The nine (dx, dy)-shifted gradient tiles are stacked along M (128/cout pairs per MMA) and the three
-// z-shifted activation tiles along N, so a stage of 64 or 128 rows is loaded once, 9 + 3 tiles, for all
-// 27 taps; plane chunks are the MN-major, no-swizzle operands as they lie (8 channels per core-matrix
-// column). Each CTA reduces a contiguous range of rows in TMEM and adds its partial weights with FP32
-// atomics. Bound by the L2 reads of the shifted tiles. Stacking taps along M only, 27 shifted tiles
-// were loaded in rows of 64, and the activations again for each MMA: 3 times the bytes in copies of
-// 1 KB by one thread. 16 -> 16 channels at 200x200x128: 2.0 ms before, 0.33 ms now (0.38 with one
-// thread issuing the copies); 64 -> 64 at 50x50x32: 0.4 ms before, 0.18; a training step of a
-// 200x200x128 volume 12.1 ms before, 4.7 ms.
+// A chunk of up to 256 rows u takes a window of the gradient rows for each dx, dy being a row offset in it, and
+// the activations at the three z shifts. The 8-channel blocks of the three windows lie one window apart and
+// are stacked along M, the z shifts along N: an MMA per dy, each dy issued by a warp of its own; plane rows are
+// the MN-major, no-swizzle operands as they lie (8 channels per core-matrix column). Each CTA reduces a
+// contiguous range of rows in TMEM and adds its partial weights with FP32 atomics, four at a time.
+// Bounds: 16 -> 16 channels move 74 KB a chunk of 256 rows from L2 (~7 TB/s in all); smaller levels wait for
+// MMAs of N = 96 and the first loads. 27 shifted tiles in rows of 64, and the activations again for each MMA,
+// took 3 times the bytes or more in copies of 1 KB. Calls, before and now: 16 -> 16 at 200x200x128 2.84 ms,
+// 0.26 ms (0.36 with chunks of 128 rows); 32 -> 32 at 100x100x64 1.02, 0.09 (0.16 with single atomics);
+// 64 -> 64 at 50x50x32 1.00, 0.07; a training step of a 200x200x128 volume 12.1 ms, 2.9 ms.
 //
 // Every mbarrier wait is bounded; a timeout sets the error flag, the roles drain what they issued
 // and the CTA frees its TMEM and returns.
@@ -535,6 +536,10 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(const ConvArgs a) {
 struct WgradArgs {
     Geom g;
     int taps, u_lo, chunks_total, chunks_per_cta, cin;
+    int kv;            // rows of a chunk
+    int segs;          // gradient copies per plane and 8 channels: one window, or the rows of dy = -1, 0, +1
+    int dy_rows, rows; // rows between the dy operands; rows of a gradient window
+    int stages;
     const __nv_bfloat16* grad;
     const __nv_bfloat16* act;
     float* dw;
@@ -543,29 +548,27 @@ struct WgradArgs {
 
 template <int COUT, int CIS>
 struct WgradCfg {
-    static constexpr int TPG = kTileM / COUT;               // (dx, dy) pairs per MMA (stacked along M)
-    static constexpr int NG = (9 + TPG - 1) / TPG;          // MMAs over the 9 pairs; the last one overlaps
-    static constexpr int KV = COUT == 16 ? 128 : 64;        // rows per stage
-    static constexpr int CHUNK = KV * 16;                   // KV rows of one 8-channel plane
-    static constexpr int ABOX = (COUT / 8) * CHUNK;         // one pair's gradient tile
-    static constexpr int BBOX = (CIS / 8) * CHUNK;          // one z shift's activation tile
-    static constexpr int STAGE = 9 * ABOX + 3 * BBOX;
+    static constexpr int CB = COUT / 8;
+    static constexpr int NB = 3 * CB;                       // 8-channel blocks of the gradient's three planes
+    static constexpr int MB = kTileM / 8;                   // blocks of an MMA
+    static constexpr int NH = NB > MB ? 2 : 1;              // MMAs over the blocks; a second one overlaps
     static constexpr int CTL = 1024;
-    static constexpr int NST_FIT = (kSmemLimit - 1024 - CTL) / STAGE;
-    static constexpr int NST = NST_FIT > 12 ? 12 : NST_FIT;
-    static constexpr int SMEM = 1024 + CTL + NST * STAGE;
-    static constexpr int TMEM_COLS = pow2_at_least(NG * 3 * CIS);
-    static_assert(NST >= 2, "wgrad: not enough shared memory for a 2-stage pipeline");
-    static_assert(SMEM <= kSmemLimit, "wgrad: shared memory over the limit");
-    static_assert(STAGE % 1024 == 0, "wgrad: stage must keep 1024-byte alignment");
-    static_assert(NG * 3 * CIS <= 512 && 3 * CIS <= 256, "wgrad: accumulators fit TMEM, N fits an MMA");
-    // first pair of MMA gi: the last one starts early enough to hold TPG pairs
-    __host__ __device__ static constexpr int pair0(int gi) { return gi * TPG + TPG <= 9 ? gi * TPG : 9 - TPG; }
+    static constexpr int TMEM_COLS = pow2_at_least(3 * NH * 3 * CIS);
+    static constexpr int THREADS = 256;
+    static_assert(3 * NH * 3 * CIS <= 512 && 3 * CIS <= 256, "wgrad: accumulators fit TMEM, N fits an MMA");
+    static_assert(NB <= NH * MB, "wgrad: the MMAs cover the blocks");
+    __host__ __device__ static int stage_bytes(int kv, int rows) { return (NB * rows + 3 * (CIS / 8) * kv) * 16; }
+    // an MMA reads MB blocks from the stage's start, whatever their number: the rows past NB are not used,
+    // but lie in the buffer
+    __host__ __device__ static int smem_bytes(int kv, int rows, int stages) {
+        const int st = stage_bytes(kv, rows), mma = MB * rows * 16;
+        return 1024 + CTL + (stages - 1) * st + (st > mma ? st : mma);
+    }
 };
 
 // Slice blockIdx.y of CIS input channels. See the file comment for the layout.
 template <int COUT, int CIS>
-__global__ void __launch_bounds__(192, 1) k_conv_wgrad(const WgradArgs a) {
+__global__ void __launch_bounds__(256, 1) k_conv_wgrad(const WgradArgs a) {
     using C = WgradCfg<COUT, CIS>;
     extern __shared__ unsigned char smem_raw[];
     const uint32_t base_addr = smem_addr(smem_raw);
@@ -576,17 +579,18 @@ __global__ void __launch_bounds__(192, 1) k_conv_wgrad(const WgradArgs a) {
     const int kz = a.taps == 27 ? 3 : 1;
     const int NN = kz * CIS;                         // MMA N: z taps stacked along N
     const int ci0 = blockIdx.y * CIS;
+    const uint32_t blk = a.rows * 16, chunk = a.kv * 16;
+    const uint32_t stage = C::stage_bytes(a.kv, a.rows);
 
     const int c_begin = blockIdx.x * a.chunks_per_cta;
     const int c_end = min(a.chunks_total, c_begin + a.chunks_per_cta);
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < C::NST; ++s) {
+        for (int s = 0; s < a.stages; ++s) {
             mbar_init(&ctl->full[s], 1);
-            mbar_init(&ctl->empty[s], 1);
+            mbar_init(&ctl->empty[s], 3);
         }
-        mbar_init(&ctl->acc_full[0], 1);
-        mbar_init(&ctl->done, 1);
+        mbar_init(&ctl->done, 3);
         ctl->abort = 0;
         mbar_init_fence();
     }
@@ -597,88 +601,99 @@ __global__ void __launch_bounds__(192, 1) k_conv_wgrad(const WgradArgs a) {
     const uint32_t tmem = uniform(ctl->tmem);
 
     if (warp == 0) {
-        const uint32_t bytes = 9 * C::ABOX + kz * C::BBOX;
-        constexpr int NA = 9 * (COUT / 8);               // gradient copies of a stage, then the activations'
+        const int seg_rows = a.segs == 1 ? a.rows : a.kv;
+        const uint32_t bytes = C::NB * blk + kz * (CIS / 8) * chunk;
+        const int NA = C::NB * a.segs;                   // gradient copies of a stage, then the activations'
         const int n_copies = NA + kz * (CIS / 8);
         int s = 0;
         unsigned ph = 0;
         long long issued = 0;
         for (int c = c_begin; c < c_end; ++c) {
-            const int u0 = a.u_lo + c * C::KV;
+            const int u0 = a.u_lo + c * a.kv;
             if (!open_stage(&ctl->empty[s], ph ^ 1, &ctl->full[s], bytes, lane, ctl, a.err)) break;
-            unsigned char* st = stages + s * C::STAGE;
+            unsigned char* st = stages + s * stage;
             for (int i = lane; i < n_copies; i += 32) {
-                const __nv_bfloat16* from;
                 if (i < NA) {
-                    const int q = i / (COUT / 8), cb = i % (COUT / 8);
-                    from = a.grad + prow(a.g, cb, u0 - (q / 3 - 1) * a.g.plane - (q % 3 - 1) * a.g.nzp);
+                    const int b = i / a.segs, j = i % a.segs;
+                    bulk_load(st + b * blk + j * chunk,
+                              a.grad + prow(a.g, b % C::CB, u0 - (b / C::CB - 1) * a.g.plane + (j - 1) * a.g.nzp),
+                              seg_rows * 16, &ctl->full[s]);
                 } else {
                     const int dz = (i - NA) / (CIS / 8), cb = (i - NA) % (CIS / 8);
-                    from = a.act + prow(a.g, ci0 / 8 + cb, u0 + dz - kz / 2);
+                    bulk_load(st + C::NB * blk + (i - NA) * chunk, a.act + prow(a.g, ci0 / 8 + cb, u0 + dz - kz / 2),
+                              chunk, &ctl->full[s]);
                 }
-                bulk_load(st + i * C::CHUNK, from, C::CHUNK, &ctl->full[s]);
             }
             ++issued;
-            if (++s == C::NST) { s = 0; ph ^= 1; }
+            if (++s == a.stages) { s = 0; ph ^= 1; }
         }
         __syncwarp();
         if (lane == 0) {
-            const long long n_drain = issued < C::NST ? issued : C::NST;
+            const long long n_drain = issued < a.stages ? issued : a.stages;
             for (long long i = 0; i < n_drain; ++i) {
-                if (--s < 0) { s = C::NST - 1; ph ^= 1; }
+                if (--s < 0) { s = a.stages - 1; ph ^= 1; }
                 mbar_wait(&ctl->full[s], ph);
             }
         }
         __syncwarp();
-    } else if (warp == 1) {
-        // MN-major, no swizzle: 8 M (or N) elements x 8 K rows per 128-byte core matrix; K groups
-        // 128 B apart (LBO), 8-element M/N blocks one chunk apart (SBO)
+    } else if (warp <= 3) {
+        // ---- MMA issuers, one for each dy. MN-major, no swizzle: 8 M (or N) elements x 8 K rows per
+        // 128-byte core matrix; K groups 128 B apart (LBO), M blocks a window apart and N blocks a chunk (SBO)
+        const int j = uniform(warp - 1);
         const uint32_t lead = elect_one();
         const uint32_t idesc = umma_idesc_bf16(kTileM, NN, true, true);
         const uint32_t sbase = smem_addr(stages);
+        const uint32_t d = tmem + j * C::NH * NN;
         int s = 0;
         unsigned ph = 0;
         for (int c = c_begin; c < c_end; ++c) {
             if (!warp_wait(&ctl->full[s], ph, ctl, a.err)) break;
             tc_fence_after();
-            const uint32_t st = sbase + s * C::STAGE;
+            const uint32_t ga = sbase + s * stage + j * a.dy_rows * 16, xa = sbase + s * stage + C::NB * blk;
+            for (int kk = 0; kk < a.kv / 16; ++kk) {
+                const uint64_t bd = umma_desc(xa + kk * 256, 128, chunk, UMMA_NONE);
 #pragma unroll
-            for (int kk = 0; kk < C::KV / 16; ++kk) {
-                const uint64_t bd = umma_desc(st + 9 * C::ABOX + kk * 256, 128, C::CHUNK, UMMA_NONE);
-#pragma unroll
-                for (int gi = 0; gi < C::NG; ++gi) {
-                    const uint64_t ad = umma_desc(st + C::pair0(gi) * C::ABOX + kk * 256, 128, C::CHUNK, UMMA_NONE);
-                    umma_bf16(tmem + gi * NN, ad, bd, idesc, (c != c_begin) || kk != 0, lead);
+                for (int h = 0; h < C::NH; ++h) {
+                    const uint64_t ad = umma_desc(ga + h * (C::NB - C::MB) * blk + kk * 256, 128, blk, UMMA_NONE);
+                    umma_bf16(d + h * NN, ad, bd, idesc, (c != c_begin) || kk != 0, lead);
                 }
             }
             umma_commit(&ctl->empty[s], lead);
-            if (++s == C::NST) { s = 0; ph ^= 1; }
+            if (++s == a.stages) { s = 0; ph ^= 1; }
         }
-        umma_commit(&ctl->acc_full[0], lead);
-        mbar_wait(&ctl->acc_full[0], 0);
+        umma_commit(&ctl->done, lead);
+        mbar_wait(&ctl->done, 0);
         __syncwarp();
     } else if (c_begin < c_end) {
         const int quad = warp & 3;
         const int row = quad * 32 + lane;
-        if (wait_or_abort(&ctl->acc_full[0], 0, ctl, a.err) && !ctl->abort) {
+        if (warp_wait(&ctl->done, 0, ctl, a.err) && !ctl->abort) {
             tc_fence_after();
-            const int j = row / COUT, co = row % COUT;
-            for (int gi = 0; gi < C::NG; ++gi) {
-                const int q = C::pair0(gi) + j;
-                const bool mine = q >= gi * C::TPG;      // not already the MMA before's
-                for (int dz = 0; dz < kz; ++dz) {
-                    float v[CIS];
+            const bool vec = reinterpret_cast<uintptr_t>(a.dw) % 16 == 0;   // a fourth of the memory operations
+            for (int j = 0; j < 3; ++j)
+                for (int h = 0; h < C::NH; ++h) {
+                    const int b = row / 8 + h * (C::NB - C::MB);
+                    const bool mine = b < C::NB && b >= h * C::MB;   // not already the MMA before's
+                    const int q = b / C::CB * 3 + 2 - j, co = b % C::CB * 8 + row % 8;
+                    for (int dz = 0; dz < kz; ++dz) {
+                        float v[CIS];
 #pragma unroll
-                    for (int c = 0; c < CIS; c += 16)
-                        tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + gi * NN + dz * CIS + c, v + c);
-                    tmem_ld_wait();
-                    if (mine) {
-                        float* dst = a.dw + ((size_t)(q * kz + dz) * COUT + co) * a.cin + ci0;
+                        for (int c = 0; c < CIS; c += 16)
+                            tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (j * C::NH + h) * NN + dz * CIS + c, v + c);
+                        tmem_ld_wait();
+                        if (mine) {
+                            float* dst = a.dw + ((size_t)(q * kz + dz) * COUT + co) * a.cin + ci0;
+                            if (vec) {
 #pragma unroll
-                        for (int c = 0; c < CIS; ++c) atomicAdd(dst + c, v[c]);
+                                for (int c = 0; c < CIS; c += 4)
+                                    atomicAdd(reinterpret_cast<float4*>(dst + c), make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]));
+                            } else {
+#pragma unroll
+                                for (int c = 0; c < CIS; ++c) atomicAdd(dst + c, v[c]);
+                            }
+                        }
                     }
                 }
-            }
         }
     }
     tc_fence_before();
@@ -782,14 +797,23 @@ template <int COUT, int CIS>
 int launch_wgrad_t(int nx, int ny, int nz, int cin, int taps, const void* grad, const void* act, float* dw,
                    cudaStream_t st, int* err, int sms) {
     using C = WgradCfg<COUT, CIS>;
-    BD_CUDA(cudaFuncSetAttribute(k_conv_wgrad<COUT, CIS>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
+    BD_CUDA(cudaFuncSetAttribute(k_conv_wgrad<COUT, CIS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
     WgradArgs a{};
     a.g = make_geom(nx, ny, nz);
     a.taps = taps;
     a.cin = cin;
+    // the longest chunks of which two stages fit: a window carries 2 nzp rows of halo
+    for (a.kv = 256;; a.kv -= 64) {
+        a.segs = a.g.nzp <= a.kv ? 1 : 3;
+        a.dy_rows = std::min(a.g.nzp, a.kv);
+        a.rows = a.kv + 2 * a.dy_rows;
+        if (a.kv == 64 || C::smem_bytes(a.kv, a.rows, 2) <= kSmemLimit) break;
+    }
+    static_assert(2 * (C::NB * 3 + 3 * (CIS / 8)) * 64 * 16 <= kSmemLimit - 2048, "wgrad: two stages of 64 rows fit");
+    for (a.stages = 2; a.stages < 6 && C::smem_bytes(a.kv, a.rows, a.stages + 1) <= kSmemLimit;) ++a.stages;
     // rows u of the sums g[u - (dx, dy)] x[u + dz]: one more on either side than the interior has
     a.u_lo = a.g.v_lo - 1;
-    a.chunks_total = (a.g.v_hi + 1 - a.u_lo + C::KV - 1) / C::KV;
+    a.chunks_total = (a.g.v_hi + 1 - a.u_lo + a.kv - 1) / a.kv;
     a.grad = static_cast<const __nv_bfloat16*>(grad);
     a.act = static_cast<const __nv_bfloat16*>(act);
     a.dw = dw;
@@ -797,10 +821,10 @@ int launch_wgrad_t(int nx, int ny, int nz, int cin, int taps, const void* grad, 
     // split the rows over the SMs; small levels keep at least 2048 rows per CTA (a CTA ends by adding
     // its 27 x cout x CIS partial weights to memory)
     const int slices = cin / CIS;
-    const int ctas = std::max(1, std::min(std::max(1, sms / slices), (a.chunks_total * C::KV + 2047) / 2048));
+    const int ctas = std::max(1, std::min(std::max(1, sms / slices), (a.chunks_total * a.kv + 2048 - 1) / 2048));
     a.chunks_per_cta = (a.chunks_total + ctas - 1) / ctas;
     const int grid = (a.chunks_total + a.chunks_per_cta - 1) / a.chunks_per_cta;
-    k_conv_wgrad<COUT, CIS><<<dim3(grid, slices), 192, C::SMEM, st>>>(a);
+    k_conv_wgrad<COUT, CIS><<<dim3(grid, slices), C::THREADS, C::smem_bytes(a.kv, a.rows, a.stages), st>>>(a);
     BD_CHECK_LAUNCH("k_conv_wgrad");
     return BD_OK;
 }
@@ -859,13 +883,13 @@ int conv_launch(const BdConvCall& c, cudaStream_t st, int* err) {
 int wgrad_launch(int nx, int ny, int nz, int cin, int cout, int taps, const void* grad, const void* act, float* dw,
                  cudaStream_t st, int* err) {
     const int sms = sm_count();
-#define BD_WG_CASE(CO, CIS_)                                                  \
-    if (cout == CO && (cin == CIS_ || (cin > CIS_ && CIS_ == 32)))            \
+#define BD_WG_CASE(CO, CIS_)                    \
+    if (cout == CO && (cin == CIS_ || (cin > CIS_ && CIS_ == (CO == 64 ? 16 : 32)))) \
         return launch_wgrad_t<CO, CIS_>(nx, ny, nz, cin, taps, grad, act, dw, st, err, sms);
-    // 64 input channels run as two slices of 32: their accumulators would not fit TMEM
+    // more input channels run as slices: their accumulators would not fit TMEM
     BD_WG_CASE(16, 16) BD_WG_CASE(16, 32)
     BD_WG_CASE(32, 16) BD_WG_CASE(32, 32)
-    BD_WG_CASE(64, 16) BD_WG_CASE(64, 32)
+    BD_WG_CASE(64, 16)
 #undef BD_WG_CASE
     return fail(BD_ERR_INVALID_ARG, "bd_conv3d_wgrad: unsupported channel combination");
 }
