@@ -37,25 +37,31 @@ __device__ __forceinline__ T block_sum(T v, T* sh) {
 }
 
 // ---- 1. phase update + removal ----------------------------------------------------------
+// Both voxel passes move 30 to 46 bytes a voxel and are bound by memory latency where loads wait for stores:
+// the fields nearly every voxel needs are loaded first, and what does not change is not stored. Together
+// 217 us at 200x200x192 with loads between the stores, 164 us now (traffic alone ~90).
 __global__ void __launch_bounds__(256) k_phase_remove(PhaseArgs a, long long nv) {
     __shared__ unsigned long long sh[8];
     unsigned long long mine = 0;
     const float t_now = a.dyn->t_now;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nv;
          i += (long long)gridDim.x * blockDim.x) {
+        // every field that most voxels need is asked for before the first use or store
         const float T = a.T[i];
-        if (a.T_peak) a.T_peak[i] = fmaxf(a.T_peak[i], T);
-        uint8_t f = a.flags[i];
-        f &= (uint8_t)~BD_FLAG_NEWLY;
+        const float peak = a.T_peak ? a.T_peak[i] : 0.0f;
+        const uint8_t was = a.flags[i];
+        const float h = a.H[i];
+        const float hl_raw = a.h_lat[i];
+        const float top = fmaxf(peak, T);
+        if (a.T_peak && __float_as_uint(top) != __float_as_uint(peak)) a.T_peak[i] = top;
+        uint8_t f = was & (uint8_t)~BD_FLAG_NEWLY;
         bool rem = false;
         if (!(f & BD_FLAG_ABLATED)) {
             if (a.single_stage) {
                 // coupled_ablation.py:61-74
-                rem = (a.H[i] >= a.h_lat[i]) && (T >= a.t_abl);
+                rem = (h >= hl_raw) && (T >= a.t_abl);
             } else {
                 bool dry = (f & BD_FLAG_DRY) != 0;
-                float h = a.H[i];
-                const float hl_raw = a.h_lat[i];
                 const float hl = fmaxf(hl_raw, 1e-30f);
                 const float dmua = gv(a.ds_mu_a, i), dk = gv(a.ds_k, i), drho = gv(a.ds_rho, i);
                 if (!dry && h > 0.0f) {
@@ -109,7 +115,7 @@ __global__ void __launch_bounds__(256) k_phase_remove(PhaseArgs a, long long nv)
             a.H[i] = 0.0f;
             ++mine;
         }
-        a.flags[i] = f;
+        if (f != was) a.flags[i] = f;
     }
     unsigned long long s = block_sum(mine, sh);
     if (threadIdx.x == 0 && s) atomicAdd(&a.dyn->n_new, s);
@@ -158,21 +164,31 @@ __global__ void __launch_bounds__(256) k_void_plume(PhaseArgs a, long long nv) {
             k -= a.nz;
             ++col;
         }
-        uint8_t f = a.flags[i];
+        // all loads before the first store: the compiler can't move one past the other
+        const uint8_t was = a.flags[i];
+        const float plume = a.has_plume ? a.plume[i] : 0.0f;
+        float ma = 0.0f, ms = 0.0f, gg = 0.0f, nn = 0.0f;
+        if (a.props) {
+            ma = a.mu_a[i];
+            ms = a.mu_s[i];
+            gg = a.g[i];
+            nn = a.n[i];
+        }
+        uint8_t f = was;
         const bool ablated = (f & BD_FLAG_ABLATED) != 0;
         const bool vd = ablated || (gap_open && k >= a.gap_k0 && k < a.gap_k1);
         f = vd ? (uint8_t)(f | BD_FLAG_VOID) : (uint8_t)(f & ~BD_FLAG_VOID);
-        a.flags[i] = f;
+        if (f != was) a.flags[i] = f;
         if (vd) {
             kmax = max(kmax, k);
             ++n_void;
         }
         float mu_ext = 0.0f;
         if (a.has_plume) {
-            float raw = a.plume[i];
+            float raw = plume;
             if (inject && (f & BD_FLAG_NEWLY)) raw = raw + a.delta_mu;   // plume.py:329
             if (!vd) raw = 0.0f;                                           // plume.py:330-331, :357-358
-            a.plume[i] = raw;
+            if (__float_as_uint(raw) != __float_as_uint(plume)) a.plume[i] = raw;
             if (vd) mu_ext = a.mu_max > 0.0f ? a.mu_max * tanhf(raw / a.mu_max) : raw;  // :359-363
             a.mu_ext[i] = mu_ext;
             const float mua_p = mu_ext * a.ratio_a;
@@ -183,14 +199,13 @@ __global__ void __launch_bounds__(256) k_void_plume(PhaseArgs a, long long nv) {
             abl_cnt += 1.0;
         }
         if (a.props) {
-            float ma = a.mu_a[i], ms = a.mu_s[i], gg = a.g[i];
             if (a.has_plume) {
                 ma = ma + mu_ext * a.ratio_a;
                 ms = ms + mu_ext * a.ratio_s;
                 if (mu_ext > 0.001f && ablated) gg = a.g_plume;
             }
             const float mt = ma + ms;
-            reinterpret_cast<float4*>(a.props)[i] = make_float4(mt, mt > 0.0f ? ma / mt : 0.0f, gg, a.n[i]);
+            reinterpret_cast<float4*>(a.props)[i] = make_float4(mt, mt > 0.0f ? ma / mt : 0.0f, gg, nn);
         }
     }
     __shared__ unsigned long long shu[8];
