@@ -18,8 +18,8 @@ ROOT = PKG.parent
 CSRC = PKG / "csrc"
 OUT_DIR = PKG / "_native"
 LIB = OUT_DIR / "libbugdef.so"
-SOURCES = ["abi.cu", "mc.cu", "stencil.cu", "plume.cu", "phase.cu", "engine.cu", "record.cu", "conv3d.cu", "unet.cu",
-           "selftest.cu"]
+SOURCES = ["abi.cu", "mc.cu", "mc_fluence.cu", "stencil.cu", "plume.cu", "phase.cu", "engine.cu", "record.cu",
+           "conv3d.cu", "unet.cu", "selftest.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

@@ -18,14 +18,15 @@
 //     and a photon's path does not depend on which thread traced it;
 //   * optical properties packed as one float4 {mu_t, mu_a/mu_t, g, n} per voxel read through
 //     the read-only (L1/texture) path: one 16-byte load per event;
-//   * absorbed weight and track length tallied with fire-and-forget reductions;
+//   * absorbed weight tallied with fire-and-forget reductions into an exact fixed-point map (launches
+//     whose sums are FP32 in memory run mc_fluence.cu's kernel);
 //   * FP64 ledger: per-thread FP64 registers for the per-event channels, per-block partial rows for
 //     the per-photon channels, reduced in a fixed order.
 // What bounds it: instructions. At 1.5 M photons about 19 warp instructions an event at 12 active
 // lanes; at 15 k the longest history (1900 events) at ~1300 clocks an event, an L2 round trip and a
 // hundred dependent instructions. Traces of the 200x200x128 stack, before the changes of this list
 // and after: 15 k photons 2.04 -> 1.40 ms, 150 k 2.95 -> 2.09 ms, 1.5 M 14.2 -> 8.6 ms; same maps.
-#include "common.cuh"
+#include "mc_dev.cuh"
 
 #include <stdlib.h>
 
@@ -34,123 +35,6 @@
 #include <mutex>
 
 namespace bd {
-
-struct McDev {
-    int nx, ny, nz, launch_axis;
-    float dx, dy, dz, lx, ly, lz;
-    float ux0, uy0, uz0, cos_ph, sin_ph, cos_th_safe;
-    float xc, yc, zc, sigma, radius;
-    int profile;
-    float n_amb, rmax2;
-    int options;
-    long long n_photons, offset;
-    unsigned max_events;
-    float fnx, fny, fnz;
-    uint32_t keys[20];   // the seed's Philox round keys
-    float eq_eps;     // Fresnel index-equality guard
-    float step_eps;   // internal index-step threshold
-    float entry_eps;  // entrance refraction threshold
-};
-
-__device__ __forceinline__ float fresnel_unpol(float n1, float n2, float cos_i, float eq_eps) {
-    // voxel_mc_3d.py:33-48 / voxel_mc_metal.py:70-83
-    if (fabsf(n1 - n2) < eq_eps) return 0.0f;
-    cos_i = fminf(1.0f, fabsf(cos_i));
-    if (cos_i > 0.999999f) {
-        float r = (n1 - n2) / (n1 + n2);
-        return r * r;
-    }
-    float q = n1 / n2;
-    float sin_t2 = q * q * (1.0f - cos_i * cos_i);
-    if (sin_t2 >= 1.0f) return 1.0f;
-    float cos_t = sqrtf(1.0f - sin_t2);
-    float a = n1 * cos_i, b = n2 * cos_t, c = n1 * cos_t, d = n2 * cos_i;
-    float rs = (a - b) / (a + b);
-    float rp = (c - d) / (c + d);
-    return 0.5f * (rs * rs + rp * rp);
-}
-
-// Snell refraction across an axis-aligned face (voxel_mc_3d.py:51-69)
-__device__ __forceinline__ void refract_axis(float& ux, float& uy, float& uz, int axis, float eta) {
-    if (axis == 0) {
-        float s = ux > 0.0f ? 1.0f : -1.0f;
-        uy *= eta; uz *= eta;
-        ux = s * sqrtf(fmaxf(0.0f, 1.0f - uy * uy - uz * uz));
-    } else if (axis == 1) {
-        float s = uy > 0.0f ? 1.0f : -1.0f;
-        ux *= eta; uz *= eta;
-        uy = s * sqrtf(fmaxf(0.0f, 1.0f - ux * ux - uz * uz));
-    } else {
-        float s = uz > 0.0f ? 1.0f : -1.0f;
-        ux *= eta; uy *= eta;
-        uz = s * sqrtf(fmaxf(0.0f, 1.0f - ux * ux - uy * uy));
-    }
-}
-
-// Henyey-Greenstein deflection + uniform azimuth (voxel_mc_3d.py:229-262); xi, xphi: uniforms
-__device__ __forceinline__ void scatter_hg(float& ux, float& uy, float& uz, float g, float xi, float xphi) {
-    float cost;
-    if (fabsf(g) < 1e-4f) {
-        cost = 2.0f * xi - 1.0f;
-    } else {
-        float t = (1.0f - g * g) / (1.0f - g + 2.0f * g * xi);
-        cost = (1.0f + g * g - t * t) / (2.0f * g);
-        cost = fminf(1.0f, fmaxf(-1.0f, cost));
-    }
-    float sint = sqrtf(fmaxf(0.0f, 1.0f - cost * cost));
-    float sinp, cosp;
-    sincospif(2.0f * xphi, &sinp, &cosp);
-    float nx, ny, nz;
-    if (fabsf(uz) > 0.99999f) {
-        float sz = uz > 0.0f ? 1.0f : -1.0f;
-        nx = sint * cosp;
-        ny = sint * sinp;
-        nz = cost * sz;
-    } else {
-        float den = sqrtf(fmaxf(1.0f - uz * uz, 1e-12f));
-        float f = sint / den;
-        nx = f * (ux * uz * cosp - uy * sinp) + ux * cost;
-        ny = f * (uy * uz * cosp + ux * sinp) + uy * cost;
-        nz = -sint * cosp * den + uz * cost;
-    }
-    float nn = nx * nx + ny * ny + nz * nz;
-    if (nn > 1e-24f) {
-        float r = rsqrtf(nn);
-        nx *= r; ny *= r; nz *= r;
-    }
-    ux = nx; uy = ny; uz = nz;
-}
-
-// Transverse launch offsets (voxel_mc_3d.py:101-120)
-__device__ __forceinline__ void beam_offsets(const McDev& P, PhotonRng& rng, float& u1, float& u2) {
-    if (P.profile == BD_BEAM_TOPHAT) {
-        float r = P.radius * sqrtf(rng.uniform(P.keys));
-        float s, c;
-        sincospif(2.0f * rng.uniform(P.keys), &s, &c);
-        u1 = r * c; u2 = r * s;
-        return;
-    }
-    if (P.profile == BD_BEAM_KIM_EXP_DISK || P.profile == BD_BEAM_KIM_GAUSS_DISK) {
-        float rn = 0.0f;
-        // rejection sampling; acceptance >= e^-2, so 256 tries all fail with p < 1e-16
-        for (int t = 0; t < 256; ++t) {
-            rn = sqrtf(rng.uniform(P.keys));
-            float acc = (P.profile == BD_BEAM_KIM_EXP_DISK) ? expf(-2.0f * rn) : expf(-2.0f * rn * rn);
-            if (rng.uniform(P.keys) < acc) break;
-        }
-        float s, c;
-        sincospif(2.0f * rng.uniform(P.keys), &s, &c);
-        u1 = P.radius * rn * c; u2 = P.radius * rn * s;
-        return;
-    }
-    // Gaussian: Box-Muller pair with per-axis sigma
-    float a = rng.uniform_pos(P.keys);
-    float b = rng.uniform(P.keys);
-    float r = sqrtf(-2.0f * logf(a)) * P.sigma;
-    float s, c;
-    sincospif(2.0f * b, &s, &c);
-    u1 = r * c; u2 = r * s;
-}
 
 // Per-thread FP64 accumulator for the per-collision channel (absorbed weight); the rare
 // channels (exits, roulette, truncation, absorption in void) go straight to the block's
@@ -261,15 +145,13 @@ __device__ __forceinline__ bool photon_launch(const McDev& P, long long pid, con
 // An interaction inside the voxel (voxel_mc_3d.py:203-262), st along the path. Returns false when the
 // photon has ended (its weight booked).
 template <int DEPTH>
-__device__ __forceinline__ bool photon_collide(const McDev& P, const uint8_t* __restrict__ flags, float* __restrict__ A,
-                                               unsigned long long* __restrict__ A64, float* __restrict__ L,
-                                               double* __restrict__ latz, double* sl, ThreadLedger& tl, PhotonState& s,
-                                               bool tally_l) {
+__device__ __forceinline__ bool photon_collide(const McDev& P, const uint8_t* __restrict__ flags,
+                                               unsigned long long* __restrict__ A64, double* __restrict__ latz, double* sl,
+                                               ThreadLedger& tl, PhotonState& s) {
     // the void flag only sorts the ledger: loaded first, used last
     const unsigned fl = flags != nullptr ? (unsigned)__ldg(&flags[s.idx]) : 0u;
     ++tl.collisions;
     const float st = s.tau / s.pr.x;
-    if (tally_l) atomicAdd(&L[s.idx], s.w * st);
     s.x += st * s.ux; s.y += st * s.uy; s.z += st * s.uz;
     if (P.rmax2 > 0.0f) {
         float a = (DEPTH == 2) ? s.x - P.xc : s.y - P.yc;
@@ -282,8 +164,7 @@ __device__ __forceinline__ bool photon_collide(const McDev& P, const uint8_t* __
     }
     const float dw = __fmul_rn(s.w, s.pr.y);
     const float w_new = __fsub_rn(s.w, dw);
-    if (A64) atomicAdd(&A64[s.idx], __float2ull_rn(dw * kTallyScale));
-    else atomicAdd(&A[s.idx], dw);
+    atomicAdd(&A64[s.idx], __float2ull_rn(dw * kTallyScale));
     const double lost = (double)s.w - (double)w_new;  // exact: both are FP32 values
     s.w = w_new;
     bool alive = true;
@@ -317,9 +198,8 @@ __device__ __forceinline__ bool photon_collide(const McDev& P, const uint8_t* __
 // the photon interacts inside the voxel first (photon_collide completes that event). Returns false
 // when the photon has ended (its weight booked).
 template <int DEPTH>
-__device__ __forceinline__ bool photon_move(const McDev& P, const float4* __restrict__ props, float* __restrict__ L,
-                                            double* __restrict__ latz, double* sl, ThreadLedger& tl, PhotonState& s,
-                                            bool metal, bool tally_l, bool& hit) {
+__device__ __forceinline__ bool photon_move(const McDev& P, const float4* __restrict__ props, double* __restrict__ latz,
+                                            double* sl, ThreadLedger& tl, PhotonState& s, bool metal, bool& hit) {
     // exact ray/box distance to the exit face (voxel_mc_3d.py:72-98)
     const float fx = s.gx + s.ox, fy = s.gy + s.oy, fz = s.gz + s.oz;
     const float sx = __fmaf_rn(fx, P.dx, -s.x) * s.iux;
@@ -338,7 +218,6 @@ __device__ __forceinline__ bool photon_move(const McDev& P, const float4* __rest
     // selection, so that lanes that cross different faces stay together ----
     ++tl.crossings;
     s.tau = __fsub_rn(s.tau, depth_out);
-    if (tally_l) atomicAdd(&L[s.idx], s.w * s_exit);
     const float ua = ax0 ? s.ux : (ax1 ? s.uy : s.uz);
     const bool fwd = ua > 0.0f;
     const float face = (ax0 ? fx : (ax1 ? fy : fz)) * (ax0 ? P.dx : (ax1 ? P.dy : P.dz));
@@ -407,9 +286,8 @@ __device__ __forceinline__ bool photon_move(const McDev& P, const float4* __rest
 #endif
 template <int DEPTH>
 __global__ void __launch_bounds__(128, BD_MC_MIN_BLOCKS) k_mc_trace(McDev P, const float4* __restrict__ props,
-                                                     const uint8_t* __restrict__ flags, float* __restrict__ A,
-                                                     unsigned long long* __restrict__ A64,
-                                                     float* __restrict__ L, double* __restrict__ latz,
+                                                     const uint8_t* __restrict__ flags,
+                                                     unsigned long long* __restrict__ A64, double* __restrict__ latz,
                                                      unsigned long long* __restrict__ queue,
                                                      double* __restrict__ partials,
                                                      const long long* __restrict__ offset_dev, int lanes) {
@@ -420,7 +298,6 @@ __global__ void __launch_bounds__(128, BD_MC_MIN_BLOCKS) k_mc_trace(McDev P, con
     tl.absorbed = tl.absorbed_void = 0.0;
     tl.collisions = tl.crossings = tl.reflections = 0u;
     const bool metal = (P.options & BD_MC_METAL_SEMANTICS) != 0;
-    const bool tally_l = (P.options & BD_MC_TALLY_FLUENCE) != 0 && L != nullptr;
 
     const unsigned long long N = (unsigned long long)P.n_photons;
     // A lane that has reached an interaction waits until half the live lanes of its warp have (or none
@@ -442,14 +319,14 @@ __global__ void __launch_bounds__(128, BD_MC_MIN_BLOCKS) k_mc_trace(McDev P, con
                 live = false;
             } else {
                 ++s.ev;
-                live = photon_move<DEPTH>(P, props, L, latz, sl, tl, s, metal, tally_l, hit);
+                live = photon_move<DEPTH>(P, props, latz, sl, tl, s, metal, hit);
             }
         }
         const unsigned wait = __ballot_sync(0xffffffffu, live && hit);
         const unsigned go = __ballot_sync(0xffffffffu, live ? !hit : more);
         if (go == 0u ? wait != 0u : 2 * __popc(wait) >= __popc(wait | go)) {
             if (live && hit) {
-                live = photon_collide<DEPTH>(P, flags, A, A64, L, latz, sl, tl, s, tally_l);
+                live = photon_collide<DEPTH>(P, flags, A64, latz, sl, tl, s);
                 hit = false;
             }
         } else if (go == 0u) {
@@ -600,6 +477,7 @@ McDev mc_dev_params(const BdMcParams* p) {
     d.n_amb = p->n_ambient; d.rmax2 = p->r_max_sq; d.options = p->options;
     d.n_photons = p->n_photons; d.offset = p->photon_offset;
     d.max_events = (unsigned)std::min<long long>(p->max_events, 0xffffffffLL);
+    d.seed = p->seed;
     d.fnx = (float)p->nx; d.fny = (float)p->ny; d.fnz = (float)p->nz;
     Philox::keys((uint32_t)p->seed, (uint32_t)(p->seed >> 32), d.keys);
     const bool metal = (p->options & BD_MC_METAL_SEMANTICS) != 0;
@@ -614,32 +492,41 @@ int mc_launch(const BdMcParams* p, const float* props, const uint8_t* flags, flo
               double* latz, double* ledger, unsigned long long* queue, double* partials, int max_blocks,
               int sm_count, cudaStream_t st, const long long* offset_dev, unsigned long long* tally64) {
     McDev d = mc_dev_params(p);
-    // resident 128-thread CTAs per SM of each kernel variant: computed once, shared by host threads
-    static std::atomic<int> per_sm[2] = {{0}, {0}};
-    const int ax = p->launch_axis == 0 ? 0 : 1;
-    int occ = per_sm[ax].load(std::memory_order_relaxed);
-    if (occ == 0) {
-        int nb = 0;
-        if (ax == 0) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_mc_trace<2>, 128, 0);
-        else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_mc_trace<0>, 128, 0);
-        occ = std::max(1, std::min(nb, 16));
-        cudaGetLastError();
-        per_sm[ax].store(occ, std::memory_order_relaxed);
-    }
-    const int want = tune_value(BD_TUNE_MC_BLOCKS_PER_SM);
-    const int use_sm = want > 0 ? std::min(want, occ) : occ;
-    // a warp runs the union of its lanes' branches, so few photons finish sooner spread over all
-    // resident warps, a few lanes of each, than packed into full ones
-    const int blocks = std::max(1, std::min((int)std::min<long long>(p->n_photons, (long long)sm_count * use_sm), max_blocks));
-    const int lanes = (int)std::min<long long>(32, std::max<long long>(1, (p->n_photons + 4LL * blocks - 1) / (4LL * blocks)));
-    BD_CUDA(cudaMemsetAsync(queue, 0, sizeof(unsigned long long), st));
-    BD_CUDA(cudaMemsetAsync(partials, 0, sizeof(double) * BD_LEDGER_LEN * blocks, st));
     const float4* pr = reinterpret_cast<const float4*>(props);
-    if (p->launch_axis == 0)
-        k_mc_trace<2><<<blocks, 128, 0, st>>>(d, pr, flags, A, tally64, L, latz, queue, partials, offset_dev, lanes);
-    else
-        k_mc_trace<0><<<blocks, 128, 0, st>>>(d, pr, flags, A, tally64, L, latz, queue, partials, offset_dev, lanes);
-    BD_CHECK_LAUNCH("k_mc_trace");
+    int blocks = 1;
+    if (((d.options & BD_MC_TALLY_FLUENCE) != 0 && L != nullptr) || tally64 == nullptr) {
+        // FP32 sums in memory depend on the order of the deposits: these launches keep the event order of
+        // mc_fluence.cu (its comment has both sides)
+        if (int rc = mc_fluence_launch(d, pr, flags, A, tally64, L, latz, queue, partials, max_blocks, sm_count, st,
+                                       offset_dev, &blocks))
+            return rc;
+    } else {
+        // resident 128-thread CTAs per SM of each kernel variant: computed once, shared by host threads
+        static std::atomic<int> per_sm[2] = {{0}, {0}};
+        const int ax = p->launch_axis == 0 ? 0 : 1;
+        int occ = per_sm[ax].load(std::memory_order_relaxed);
+        if (occ == 0) {
+            int nb = 0;
+            if (ax == 0) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_mc_trace<2>, 128, 0);
+            else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_mc_trace<0>, 128, 0);
+            occ = std::max(1, std::min(nb, 16));
+            cudaGetLastError();
+            per_sm[ax].store(occ, std::memory_order_relaxed);
+        }
+        const int want = tune_value(BD_TUNE_MC_BLOCKS_PER_SM);
+        const int use_sm = want > 0 ? std::min(want, occ) : occ;
+        // a warp runs the union of its lanes' branches, so few photons finish sooner spread over all
+        // resident warps, a few lanes of each, than packed into full ones
+        blocks = std::max(1, std::min((int)std::min<long long>(p->n_photons, (long long)sm_count * use_sm), max_blocks));
+        const int lanes = (int)std::min<long long>(32, std::max<long long>(1, (p->n_photons + 4LL * blocks - 1) / (4LL * blocks)));
+        BD_CUDA(cudaMemsetAsync(queue, 0, sizeof(unsigned long long), st));
+        BD_CUDA(cudaMemsetAsync(partials, 0, sizeof(double) * BD_LEDGER_LEN * blocks, st));
+        if (p->launch_axis == 0)
+            k_mc_trace<2><<<blocks, 128, 0, st>>>(d, pr, flags, tally64, latz, queue, partials, offset_dev, lanes);
+        else
+            k_mc_trace<0><<<blocks, 128, 0, st>>>(d, pr, flags, tally64, latz, queue, partials, offset_dev, lanes);
+        BD_CHECK_LAUNCH("k_mc_trace");
+    }
     if (tally64) {
         const long long nv = (long long)p->nx * p->ny * p->nz;
         k_tally_finalize<<<grid_for(nv, 256), 256, 0, st>>>(tally64, A, nv);
