@@ -50,8 +50,8 @@ def parse():
     ap.add_argument("--no-autotune", action="store_true")
     ap.add_argument("--no-full-run", action="store_true", help="skip the device-timed 1000-epoch schedule")
     ap.add_argument("--plume-kernel", type=int, default=None, choices=[4, 6],
-                    help="plume kernel to use (4 direct, 6 direct over a compact unit list) instead of "
-                         "the autotuner's choice")
+                    help="plume kernel to use (4 the whole stage in one launch, 6 a launch per step over a "
+                         "compact unit list) instead of the autotuner's choice")
     ap.add_argument("--batch-plume", action="store_true",
                     help="campaign: run the instances' plume stages as one batched stage (one launch per step)")
     ap.add_argument("--workload", default="coupled", choices=["coupled", "campaign"],
@@ -228,7 +228,7 @@ def make_engine(geo, dev, seed_offset=0):
 
 
 def algorithmic_bytes(eng, n_void):
-    """Unique bytes each stage must move per launch (cache-ideal neighbours)."""
+    """Unique bytes each stage must move per substep or plume step (cache-ideal neighbours)."""
     nv = eng.Nx * eng.Ny * eng.Nz
     # fused substep over every voxel: T r+w 8, k 4, rho 4, source 4, flags 1, H r+w 8, chi r+w 8
     sub = nv * 37
@@ -421,6 +421,8 @@ def ours_main(args):
             "units_per_launch": ("voxel-substeps" if dom == "substeps" else "plume (void) voxel-steps"),
             "void_voxels": int(n_void)}
     if dom == "plume":
+        if plume_kernel == "k_plume_chain":
+            roof["launch"] = "one launch runs the stage; bytes and ms are a step's"
         l2 = l2_copy_gbs(eng.dev)
         roof.update({"l2_peak": round(l2, 1), "l2_frac": round(achieved / l2, 4),
                      "l2_method": "best of 8, 16 and 32 MB device-to-device copies (L2-resident pairs), 100 "
@@ -453,11 +455,11 @@ def ours_main(args):
             mc["issue_roof_photon_steps_per_s"] = roof_steps
             mc["issue_roof_frac"] = round(mc["photon_steps_per_s"] / roof_steps, 4)
             mc["thread_instructions_per_photon_step"] = ipp
-    # per epoch: begin + 3 epoch-end kernels + the plume stage's set-up (mask and z lists; with the
-    # compact kernel the mask, bitmaps, unit counts, x-planes pick, z lists and unit list) + substeps +
-    # plume steps; per laser epoch: MC, ledger reduction and tally finalisation
-    plume_prep = 6 if kv.value == _lib.PLUME_KERNEL_COMPACT else 2
-    gpu_launches = K * (1 + 3 + plume_prep + eng.n_substeps + eng.n_substeps * n_plume_sub) + r["n_on"] * 3
+    # per epoch: begin + 3 epoch-end kernels + substeps + the plume stage (mask, bitmaps, units and one
+    # launch for all steps; with the compact kernel the mask, bitmaps, unit counts, x-planes pick, z lists
+    # and unit list, then a launch per step); per laser epoch: MC, ledger reduction and tally finalisation
+    plume_launches = 6 + eng.n_substeps * n_plume_sub if kv.value == _lib.PLUME_KERNEL_COMPACT else 4
+    gpu_launches = K * (1 + 3 + plume_launches + eng.n_substeps) + r["n_on"] * 3
     out = {"metric": METRIC, "value": round(value, 3), "unit": "epochs/s", "n_gpus": world, "steps": K,
            "warmup": args.warmup, "ms_per_step": round(ms / K, 4), "higher_is_better": True, "scaling": "weak",
            "vs_baseline": None, "dtype": "f32 (FP64 ledgers)", "data": "synthetic (seeded, reference config shapes)",
