@@ -1,4 +1,4 @@
-// Self-test of the failure path every TMA-fed kernel relies on: a bounded mbarrier wait that runs
+// Self-test of the failure path every kernel with mbarrier waits relies on: a bounded mbarrier wait that runs
 // out reports a status the host reads, and the context stays usable afterwards. No counterpart in
 // the reference. The kernel waits, through the same bounded-wait routine the kernels use, on an
 // mbarrier that nothing arrives on (arrive = 0) or that it has completed itself (arrive = 1).

@@ -374,7 +374,7 @@ BD_API int bd_engine_record(BdEngine* e, const BdRecordSpec* spec, void* slot, v
  * change bumps a generation counter so engines re-capture their epoch graphs. */
 #define BD_TUNE_MC_BLOCKS_PER_SM  0  /* persistent MC grid: 128-thread CTAs per SM, 1..16 (0 = occupancy
                                         limit); photons per thread = n_photons / (grid * 128)          */
-#define BD_TUNE_STENCIL_XC        1  /* x-planes per CTA of the TMA substep kernel, 1..64 (default 8)   */
+#define BD_TUNE_STENCIL_XC        1  /* most x-planes per CTA of the substep kernel, 1..64 (default 8)   */
 #define BD_TUNE_PLUME_XC          2  /* batched plume stage: x-planes per unit, 1..64 (default 4)       */
 #define BD_TUNE_PLUME_KERNEL      3  /* plume stage: BD_PLUME_KERNEL_DIRECT (default) or
                                         BD_PLUME_KERNEL_COMPACT (value 5 is not used)                   */
