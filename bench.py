@@ -538,8 +538,8 @@ def denoised_run_leg(n_laser=10, check_every=5):
         row["speedup"] = round(row["plain_ms_per_laser_epoch"] / row["denoised_ms_per_laser_epoch"], 3)
         out.append(row)
     return {"runs": out, "laser_epochs_timed": n_laser,
-            "note": "laser-on epochs of the full-resolution coupled run; the plume stage (one launch per FTCS "
-                    "step, beside MC and the substeps) bounds the epoch, so a cheaper optical step shortens "
+            "note": "laser-on epochs of the full-resolution coupled run; the plume stage (one launch for all "
+                    "its FTCS steps, beside MC and the substeps) bounds the epoch, so a cheaper optical step shortens "
                     "the epoch only by what it removes from the plume stream's competition"}
 
 
