@@ -12,8 +12,10 @@
 // whole 16-byte rows. The plane x adds to the outputs of x-1, x and x+1 at once: the three are neighbours in
 // TMEM and stacked along N, one 128 x 48 x 16 MMA per (dy, dz) and K step, and the weights lie in shared
 // memory so that every rotation of the three slots is a run. Each z tap has accumulators of its own, summed
-// as (t0 + t-1) + t+1 at the end, which keeps the sums' order of 27 taps as (dx, dy) runs. A finished output
-// plane's slot is read, cleared for the plane three on, and goes through the fused epilogue (bias, ReLU,
+// over (dx, dy) in order, and the three are added at the end: (t0 + t-1) + t+1, but the third before the second
+// in 3 of 126 rows, which is the order of the kernel before (its tiles of 126 outputs crossed warps there), so
+// that stored weights give the same maps to the last bit: a bf16 rounding that flips at a coarse level moves
+// the map by up to 0.2 % around it. A finished output plane's slot is read, cleared for the plane three on, and goes through the fused epilogue (bias, ReLU,
 // nearest upsampling with the skip add, gradient gating, the 1x1 head), a group of 4 warps per tile. Three
 // warps issue MMAs, one a tile: the tensor pipe queues only a few, and a warp that waits for its barrier
 // leaves it idle for hundreds of clocks.
@@ -326,27 +328,31 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv(const ConvArgs a) {
     if (threadIdx.x < kSlice)
         sbias[threadIdx.x] = (a.mode <= BD_CONV_FWD_HEAD && a.bias) ? a.bias[n0 + threadIdx.x] : 0.f;
     if (warp == 1) tmem_alloc(&ctl->tmem, 512);
-    // resident weights, wsm[dy][dz][k plane][5 dx][16 outputs][8], by plain loads: a bulk copy takes ~100
-    // clocks to issue whatever its size, and these would be 256-byte ones
-    for (int i = threadIdx.x; i < 3 * kz * C::KP * 5 * kSlice; i += kConvThreads) {
-        const int n = i % kSlice, blk = i / kSlice % 5, r = i / kSlice / 5, kp = r % C::KP, t = r / C::KP;
-        const int dz = t % kz, dy = t / kz, dx = 2 - blk % 3;       // 2, 1, 0 = +1, 0, -1
-        reinterpret_cast<uint4*>(wsm)[i] = *reinterpret_cast<const uint4*>(
-            a.wimage + ((((dx * 3 + dy) * C::KP + kp) * kz + dz) * a.n_slice + n0 + n) * 8);
-    }
-    fence_proxy_async_smem();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = uniform(ctl->tmem);
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;      // TMEM lanes of an epilogue warp
-    if (warp >= 4 && warp < 8) {
-        for (int c = 0; c < kMaxTiles * kTileCols; c += 16) tmem_zero16(tmem + lanes + c);
-        tmem_st_wait();
+    if (warp != 0) {
+        // While the producer fetches the first planes (a 40x48x52 map 144 us, 149 one after the other): clear
+        // the accumulators, and bring the resident weights, wsm[dy][dz][k plane][5 dx][16 outputs][8], by plain
+        // loads (as bulk copies, 256 bytes each at ~100 clocks to issue, they took 8 us a launch).
+        if (warp >= 4 && warp < 8) {
+            for (int c = 0; c < kMaxTiles * kTileCols; c += 16) tmem_zero16(tmem + lanes + c);
+        }
+#pragma unroll 4
+        for (int i = threadIdx.x - 32; i < 3 * kz * C::KP * 5 * kSlice; i += kConvThreads - 32) {
+            const int n = i % kSlice, blk = i / kSlice % 5, r = i / kSlice / 5, kp = r % C::KP, t = r / C::KP;
+            const int dz = t % kz, dy = t / kz, dx = 2 - blk % 3;       // 2, 1, 0 = +1, 0, -1
+            reinterpret_cast<uint4*>(wsm)[i] = __ldg(reinterpret_cast<const uint4*>(
+                a.wimage + ((((dx * 3 + dy) * C::KP + kp) * kz + dz) * a.n_slice + n0 + n) * 8));
+        }
+        if (warp >= 4 && warp < 8) tmem_st_wait();
+        fence_proxy_async_smem();
+        tc_fence_before();
+        asm volatile("bar.sync 1, %0;" ::"n"(kConvThreads - 32) : "memory");
+        tc_fence_after();
     }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
 
     if (warp == 0) {
         // ---- producer: the units' planes x0-1 .. x1+1 one after another ----
@@ -730,8 +736,9 @@ __global__ void k_pack_weights(int taps, int cin, int cout, int n_off, int n_sli
 }
 
 // Units of k_conv, by the clocks of a CTA: a tile's MMAs at ~75 clocks each with their waits, or its epilogue
-// (~650), and a plane's load at ~24 bytes a clock; fits 43 to 75 give the same times to 2%. A unit reads two planes more than it writes, and a short group its dy halo too
-// often; the units should fill the CTAs evenly.
+// (~650), and a plane's load at ~24 bytes a clock (43 to 75 clocks an MMA give the same times to 3 %). A unit
+// reads two planes more than it writes, and a short group its dy halo too often; the units should fill the
+// CTAs evenly.
 MarchPlan march_plan(const Geom& g, int cin, int taps, int avail, int ctas) {
     const int nx = g.nxp - 2, in_rows = (g.nyp - 2) * g.nzp - 2;
     const double tile_clk = std::max(650.0, 75.0 * (taps / 3) * (cin / 16));

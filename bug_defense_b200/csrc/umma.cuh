@@ -49,9 +49,9 @@ __device__ __forceinline__ uint32_t elect_one() {
 // The value lane 0 holds, known to be the same in the whole warp.
 __device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
 
-// D[tmem] (+)= A[smem] * B[smem]^T, issued by the lane with lead != 0. The whole warp calls it: operands that
-// every lane computes alike stay in uniform registers, which is where the instruction takes them from; a loop
-// that only one lane runs moves each of them over, ~100 clocks per MMA.
+// D[tmem] (+)= A[smem] * B[smem]^T, issued by the lane with lead != 0 (0 elsewhere); the whole warp calls it, so
+// that operands which every lane computes alike stay in uniform registers. A 128 x N x 16 MMA takes 43 clocks up
+// to N = 48, with either operand's rows at any 16-byte offset.
 __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                           bool accumulate, uint32_t lead) {
     asm volatile(
