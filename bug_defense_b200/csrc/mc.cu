@@ -53,13 +53,17 @@ struct PhotonState {
     PhotonRng rng;
     float x, y, z, ux, uy, uz;
     float iux, iuy, iuz;   // 1 / u, or 1 along an axis the photon does not move on
-    float gx, gy, gz;      // voxel indices (small whole numbers, exact in FP32)
+    float gx, gy, gz;      // voxel indices (whole numbers up to kMcMaxAxis, exact in FP32)
     float ox, oy, oz;      // the exit face's offset from them: 1 or 0 by direction, kFar when not moving
     float tau, w;
     float4 pr;
     int idx;
     unsigned ev;
 };
+
+// The longest axis whose indices, and the one past its end, are exact in FP32: beyond it gx + 1 == gx, and
+// the photon's linear index would walk out of the grid unseen.
+constexpr int kMcMaxAxis = 1 << 24;
 
 // Puts the exit face of an axis without motion out of reach: its distance is about 1e30 voxels.
 constexpr float kFar = 1e30f;
@@ -494,7 +498,9 @@ int mc_launch(const BdMcParams* p, const float* props, const uint8_t* flags, flo
     McDev d = mc_dev_params(p);
     const float4* pr = reinterpret_cast<const float4*>(props);
     int blocks = 1;
-    if (((d.options & BD_MC_TALLY_FLUENCE) != 0 && L != nullptr) || tally64 == nullptr) {
+    // k_mc_trace tests the bounds on voxel indices in FP32, exact up to 2^24; mc_fluence.cu's are integers
+    const bool long_axis = std::max(p->nx, std::max(p->ny, p->nz)) > kMcMaxAxis;
+    if (((d.options & BD_MC_TALLY_FLUENCE) != 0 && L != nullptr) || tally64 == nullptr || long_axis) {
         // FP32 sums in memory depend on the order of the deposits: these launches keep the event order of
         // mc_fluence.cu (its comment has both sides)
         if (int rc = mc_fluence_launch(d, pr, flags, A, tally64, L, latz, queue, partials, max_blocks, sm_count, st,

@@ -1,5 +1,6 @@
 // Photon tracer of the launches whose results are FP32 sums in memory: the track length (fluence), and the
-// absorbed map where no exact tally is kept.
+// absorbed map where no exact tally is kept; and of grids with an axis of more than 2^24 voxels, whose
+// indices mc.cu's FP32 cannot hold.
 //
 // An FP32 sum of thousands of deposits depends on their order by up to 3e-6 of the map (2-norm, 75 k photons on
 // a 26x40x50 grid): the beam's voxels first take the photons' equal first chords. Two traces with this order
