@@ -504,6 +504,8 @@ extern "C" int bd_plume_batch_create(BdEngine* const* engines, int n, BdPlumeBat
         BD_REQUIRE(p.nx == p0.nx && p.ny == p0.ny && p.nz == p0.nz && p.dx == p0.dx && p.dy == p0.dy && p.dz == p0.dz,
                    "bd_plume_batch_create: engine %d has another grid", i);
         BD_REQUIRE(p.nz % 4 == 0 && p.nz <= 1020, "bd_plume_batch_create: needs nz %% 4 == 0 and nz <= 1020");
+        BD_REQUIRE(bd::plume_aligned(e->d.phase.plume, e->d.plume_alt),
+                   "bd_plume_batch_create: engine %d's plume buffers must be 16-byte aligned", i);
     }
     BdPlumeBatch* b = new BdPlumeBatch();
     b->order.resize(n);

@@ -58,6 +58,10 @@ int ablation_launch(const BdAblationParams* p, float* Ta, float* Tb, int n, floa
                     const uint8_t* F, const float* src, const float* K, const float* R, cudaStream_t st);
 int plume_launch(const BdPlumeParams* p, float* Ca, float* Cb, int n_substeps, const uint8_t* F, int* in_b,
                  cudaStream_t st, const int* zlimit, int full_first, uint8_t* mask, int* err);
+// Whether both buffers of a plume field take float4 accesses.
+inline bool plume_aligned(const float* Ca, const float* Cb) {
+    return ((reinterpret_cast<uintptr_t>(Ca) | reinterpret_cast<uintptr_t>(Cb)) & 15) == 0;
+}
 int plume_policy_steps(const BdPlumeParams* p, int* n_steps, float* dt_step, float* decay_step);
 // One instance of a batched plume stage (several engines' plume stages in one launch per step).
 struct PlumeTab;

@@ -1085,7 +1085,7 @@ int plume_launch(const BdPlumeParams* p, float* Ca, float* Cb, int n_substeps, c
     }
     const long long total = (long long)steps * n_substeps;
     const int kernel = tune_value(BD_TUNE_PLUME_KERNEL);
-    const bool vec = nz % 4 == 0;  // rows of whole float4 groups
+    const bool vec = nz % 4 == 0 && plume_aligned(Ca, Cb);  // rows of whole float4 groups
     if (kernel == BD_PLUME_KERNEL_COMPACT && vec && (nz + 3) / 4 <= 255) {
         const int n_yt = (ny + PD_BY - 1) / PD_BY;
         unsigned* hdr = reinterpret_cast<unsigned*>(mask + plume_units_offset(nx, ny, nz));

@@ -218,7 +218,8 @@ BD_API int bd_ablation_advance(const BdAblationParams* p, float* T_a, float* T_b
 /* ---- plume diffusion (plume.py:18-80; Metal block metal_ablation_solver.py:193-240) --- */
 /* Advances n_substeps thermal substeps of plume transport in the BD_FLAG_VOID domain;
  * each substep is 1 step (AS_GIVEN, METAL) or n_sub steps (SUBCYCLE). Result lands in
- * *result_in_b = 0 -> C_a, 1 -> C_b (host int written synchronously from the step count). */
+ * *result_in_b = 0 -> C_a, 1 -> C_b (host int written synchronously from the step count).
+ * C_a and C_b may lie at any float address; 16-byte aligned ones are moved four voxels at a time. */
 BD_API int bd_plume_advance(const BdPlumeParams* p, float* C_a, float* C_b, int n_substeps,
                      const uint8_t* flags, int* result_in_b, void* stream);
 /* Number of plume steps per substep the parameters imply (SUBCYCLE: ceil of dt/dt_stable). */
@@ -314,7 +315,8 @@ BD_API int bd_engine_epoch_finish(BdEngine* e, void* stream);
  * run_highres_knowledge_suite.py:633-654). The engines' epochs are enqueued with
  * BD_EPOCH_EXTERNAL_PLUME; bd_plume_batch_run then advances every engine's plume field over one epoch
  * (its results are those of each engine's own stage), after which each engine's epoch end is
- * enqueued with bd_engine_epoch_finish. The stage runs as a CUDA graph captured on the first call. */
+ * enqueued with bd_engine_epoch_finish. The stage runs as a CUDA graph captured on the first call.
+ * The engines' plume buffers must be 16-byte aligned. */
 typedef struct BdPlumeBatch BdPlumeBatch;
 BD_API int bd_plume_batch_create(BdEngine* const* engines, int n, BdPlumeBatch** out);
 BD_API int bd_plume_batch_run(BdPlumeBatch* b, void* stream);
