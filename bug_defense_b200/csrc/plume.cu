@@ -7,7 +7,9 @@
 //                     pass over the field
 //   k_plume_direct_c  (BD_PLUME_KERNEL_COMPACT): one launch per step, one wave of CTAs looping over a
 //                     compact list of the live units, x planes per unit chosen per stage
-//   k_plume_step      grids of more than 255 z groups (nz > 1020): one voxel per thread
+//   k_plume_direct    grids of more than 255 z groups (nz > 1020) in whole, aligned float4 rows: one launch
+//                     per step, a CTA per 32 (z) x 16 (y) tile column
+//   k_plume_step      the other grids of more than 255 z groups: one voxel per thread
 // Layout: C-order (nx, ny, nz), z fastest; the neighbourhood of every voxel is one mask byte.
 #include "common.cuh"
 #include "engine.cuh"
@@ -203,7 +205,7 @@ __global__ void __launch_bounds__(PM_TZ * PM_TY) k_plume_step(int nx, int ny, in
     }
 }
 
-// ---- one step per launch: the units of the compact and the batched kernel ---------------------
+// ---- one step per launch: the units of the direct, the compact and the batched kernel ----------
 // A unit is 16 rows (y) by 8 live z groups and marches xc x planes; thread = 4 consecutive z voxels of
 // one row, a warp 8 such groups x 4 rows (one 128-byte line per row and load). The thread keeps the
 // x-1 / x float4 of its row in registers and loads, per plane, the next plane's float4 and the
@@ -333,6 +335,21 @@ __device__ __forceinline__ void plume_direct_unit(const float* __restrict__ C, f
     const int zg = threadIdx.x & 7;
     const int g = b0 + zg < cnt ? (int)zlist[n_cols + col * G + b0 + zg] : -2;
     plume_unit_groups(C, Cn, M, nx, ny, nz, mz, xc, k, zl, g, yt, xch, w0s);
+}
+
+// One step over a grid of units: blockIdx = (band of 8 consecutive z groups, y tile, x chunk). For grids whose z
+// groups exceed a list's one-byte ids. 64 x 64 x 1200, 680 steps: 7.0 ms a call, 14.0 ms by one voxel per thread.
+__global__ void __launch_bounds__(8 * PD_BY, 9) k_plume_direct(const float* __restrict__ C, float* __restrict__ Cn,
+                                                               const uint8_t* __restrict__ M, int nx, int ny, int nz,
+                                                               int mz, int xc, const __grid_constant__ PlumeTab k,
+                                                               const int* __restrict__ zlimit) {
+    __shared__ float w0s[64];
+    if (threadIdx.x < 64) w0s[threadIdx.x] = k.w0eff[threadIdx.x];
+    __syncthreads();
+    const int zl = zlimit ? min(max(*zlimit, 0), nz) : nz;
+    const int g0 = 8 * (int)blockIdx.x, g = g0 + (threadIdx.x & 7);
+    if (4 * g0 >= zl) return;  // uniform over the CTA
+    plume_unit_groups(C, Cn, M, nx, ny, nz, mz, xc, k, zl, 4 * g < zl ? g : -2, blockIdx.y, blockIdx.z, w0s);
 }
 
 // ---- BD_PLUME_KERNEL_COMPACT: a compact list of live units, one launch per step --------------
@@ -1135,11 +1152,17 @@ int plume_launch(const BdPlumeParams* p, float* Ca, float* Cb, int n_substeps, c
         if (in_b) *in_b = flips & 1;
         return BD_OK;
     }
+    const int xc = tune_value(BD_TUNE_PLUME_XC);
+    const dim3 dgrid((nz + 31) / 32, (ny + PD_BY - 1) / PD_BY, (nx + xc - 1) / xc);
+    const bool direct = vec && dgrid.y <= 65535;
     for (long long s = 0; s < total; ++s) {
         const float* in = (s & 1) ? Cb : Ca;
         float* out = (s & 1) ? Ca : Cb;
-        k_plume_step<<<dim3((ny + PM_TY - 1) / PM_TY, nx), dim3(PM_TZ, PM_TY), 0, st>>>(nx, ny, nz, mz, tab, in, out, mask,
-                                                                                        zl);
+        if (direct)
+            k_plume_direct<<<dgrid, 8 * PD_BY, 0, st>>>(in, out, mask, nx, ny, nz, mz, xc, tab, zl);
+        else
+            k_plume_step<<<dim3((ny + PM_TY - 1) / PM_TY, nx), dim3(PM_TZ, PM_TY), 0, st>>>(nx, ny, nz, mz, tab, in, out,
+                                                                                            mask, zl);
     }
     BD_CHECK_LAUNCH("k_plume_step");
     if (in_b) *in_b = (int)(total & 1);

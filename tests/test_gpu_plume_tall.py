@@ -1,0 +1,68 @@
+"""Plume grids of more than 255 z groups (nz > 1020), one launch per step, against the FP64 oracle: rows of
+whole float4 groups by k_plume_direct, the others by k_plume_step. Ragged y tiles and x chunks, a last band of
+fewer than 8 groups, single planes and rows.
+
+Tolerance: FP32 against FP64, each step a convex combination rounded a few times: the relative error stays below
+(steps) x 8 x 2^-24."""
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _advance(shape, vd, C0, steps, dx, dy, dz, dt, Dxy, Dz, vz, tau):
+    import torch
+    from bug_defense_b200 import _lib
+    from bug_defense_b200.ablation import plume_params_struct
+    a = torch.from_numpy(C0).cuda()
+    b = torch.full_like(a, 7.0)
+    flags = torch.from_numpy((vd * _lib.FLAG_VOID).astype(np.uint8)).cuda()
+    p = plume_params_struct(shape, dx, dy, dz, dt, Dxy, Dz, vz, tau, "as_given")
+    in_b = ctypes.c_int(0)
+    _lib.call("bd_plume_advance", ctypes.byref(p), _lib.ptr(a), _lib.ptr(b), steps, _lib.ptr(flags), ctypes.byref(in_b),
+              _lib.stream_ptr())
+    return (b if in_b.value else a).cpu().numpy()
+
+
+@pytest.mark.parametrize("shape,kind", [((9, 21, 1024), "pores"), ((6, 17, 1028), "layers"), ((5, 16, 1021), "pores"),
+                                        ((7, 19, 1201), "layers"), ((3, 3, 2052), "full"), ((1, 5, 1024), "full"),
+                                        ((5, 1, 1023), "full")])
+def test_tall_grids_match_oracle(gpu, orc, shape, kind):
+    rng = np.random.default_rng(sum(shape))
+    vd = rng.uniform(size=shape) < 0.8
+    if kind == "full":
+        vd[:] = True
+    elif kind == "layers":
+        vd[:] = False
+        vd[:, :, :shape[2] // 3] = True
+        vd[:, :, shape[2] - 7:] = True
+    C0 = (rng.uniform(0.1, 1.0, shape)).astype(np.float32)      # non-void voxels may hold anything
+    args = (0.03, 0.025, 0.02, 1e-5, 1.5, 2.5, 4.0)
+    for steps in (1, 6, 25):
+        got = _advance(shape, vd, C0, steps, *args, 0.02)
+        C, Cn = np.where(vd, C0, 0.0).astype(np.float64), np.empty(shape)
+        for _ in range(steps):
+            orc.diffuse_plume_step(C, Cn, vd, *shape, *args, float(np.exp(-1e-5 / 0.02)))
+            C, Cn = Cn, C
+        np.testing.assert_allclose(got, C, rtol=steps * 8 * 2.0 ** -24, atol=1e-12, err_msg=f"{steps} steps")
+        assert np.all(got[~vd] == 0.0)
+
+
+@pytest.mark.parametrize("nz,kernel", [(1024, "k_plume_direct"), (1020, "k_plume_chain"), (1025, "k_plume_step")])
+def test_kernel_of_a_tall_grid(gpu, nz, kernel):
+    """Whole float4 rows are moved four voxels at a time whatever their length: one voxel per thread takes twice as
+    long."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+    rng = np.random.default_rng(nz)
+    shape = (6, 20, nz)
+    C0 = rng.uniform(0.1, 1.0, shape).astype(np.float32)
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        _advance(shape, np.ones(shape, bool), C0, 400, 0.03, 0.025, 0.02, 1e-5, 1.5, 2.5, 4.0, 0.02)
+        torch.cuda.synchronize()
+    names = {e.key for e in prof.key_averages()}
+    ran = {n for n in ("k_plume_direct", "k_plume_chain", "k_plume_step")
+           if any(f"::{n}(" in key or f"::{n}<" in key for key in names)}
+    assert ran == {kernel}, names
