@@ -3,13 +3,14 @@
 // centre), Dirichlet 0 on the outer walls, clamped at 0, optional first-order decay.
 //
 // Kernels (all evaluate the same per-voxel expression, ftcs1 / ftcs4, so they are bit-identical):
-//   k_plume_chain     default (BD_PLUME_KERNEL_DIRECT): a whole stage in one launch, 4 FTCS steps per
+//   k_plume_chain     BD_PLUME_KERNEL_DIRECT, the default: a whole stage in one launch, 4 FTCS steps per
 //                     pass over the field
+//   k_plume_direct    the default's stages of too few steps for a chain (chain_pays), and grids of more than
+//                     255 z groups (nz > 1020): one launch per step, a CTA per 32 (z) x 16 (y) tile column;
+//                     whole, aligned float4 rows
+//   k_plume_step      the same for other rows: one voxel per thread
 //   k_plume_direct_c  (BD_PLUME_KERNEL_COMPACT): one launch per step, one wave of CTAs looping over a
 //                     compact list of the live units, x planes per unit chosen per stage
-//   k_plume_direct    grids of more than 255 z groups (nz > 1020) in whole, aligned float4 rows: one launch
-//                     per step, a CTA per 32 (z) x 16 (y) tile column
-//   k_plume_step      the other grids of more than 255 z groups: one voxel per thread
 // Layout: C-order (nx, ny, nz), z fastest; the neighbourhood of every voxel is one mask byte.
 #include "common.cuh"
 #include "engine.cuh"
@@ -337,19 +338,27 @@ __device__ __forceinline__ void plume_direct_unit(const float* __restrict__ C, f
     plume_unit_groups(C, Cn, M, nx, ny, nz, mz, xc, k, zl, g, yt, xch, w0s);
 }
 
-// One step over a grid of units: blockIdx = (band of 8 consecutive z groups, y tile, x chunk). For grids whose z
-// groups exceed a list's one-byte ids. 64 x 64 x 1200, 680 steps: 7.0 ms a call, 14.0 ms by one voxel per thread.
+// One step over a grid of units: blockIdx = (band, y tile, x chunk), the bands from the columns' z lists, or of
+// 8 consecutive z groups where there are none (nz > 1020: a group's id is a byte in a list; 64 x 64 x 1200, 680
+// steps: 7.0 ms a call, 14.0 ms by one voxel per thread).
+template <bool LISTED>
 __global__ void __launch_bounds__(8 * PD_BY, 9) k_plume_direct(const float* __restrict__ C, float* __restrict__ Cn,
                                                                const uint8_t* __restrict__ M, int nx, int ny, int nz,
                                                                int mz, int xc, const __grid_constant__ PlumeTab k,
-                                                               const int* __restrict__ zlimit) {
+                                                               const int* __restrict__ zlimit,
+                                                               const uint8_t* __restrict__ zlist) {
     __shared__ float w0s[64];
     if (threadIdx.x < 64) w0s[threadIdx.x] = k.w0eff[threadIdx.x];
     __syncthreads();
     const int zl = zlimit ? min(max(*zlimit, 0), nz) : nz;
-    const int g0 = 8 * (int)blockIdx.x, g = g0 + (threadIdx.x & 7);
-    if (4 * g0 >= zl) return;  // uniform over the CTA
-    plume_unit_groups(C, Cn, M, nx, ny, nz, mz, xc, k, zl, 4 * g < zl ? g : -2, blockIdx.y, blockIdx.z, w0s);
+    if (LISTED) {
+        plume_direct_unit(C, Cn, M, nx, ny, nz, mz, xc, k, zl, zlist, gridDim.y * gridDim.z,
+                          blockIdx.z * gridDim.y + blockIdx.y, blockIdx.y, blockIdx.z, blockIdx.x, w0s);
+    } else {
+        const int g0 = 8 * (int)blockIdx.x, g = g0 + (threadIdx.x & 7);
+        if (4 * g0 >= zl) return;  // uniform over the CTA
+        plume_unit_groups(C, Cn, M, nx, ny, nz, mz, xc, k, zl, 4 * g < zl ? g : -2, blockIdx.y, blockIdx.z, w0s);
+    }
 }
 
 // ---- BD_PLUME_KERNEL_COMPACT: a compact list of live units, one launch per step --------------
@@ -1036,6 +1045,35 @@ static cudaError_t chain_blocks(int S, int slots, float* Ca, float* Cb, const ui
     }
 }
 
+// Whether a stage of `total` steps is shorter as a chain than as a launch per step. A chain marches along all of x
+// before its first block of 4 steps is done, and once more for a remainder of 1 to 3 steps, on one SM per 16 rows;
+// a launch per step has a fixed cost and then the voxels'. Estimates in us, set so that they cross where the measured
+// times do. A step in a captured stage: 4.2 + 0.7 a million voxels (3.1 to 11.6 in all, by the depth of the void
+// domain), scalar rows 3.3 + 1.8 (1.9 to 18). `whole`: launched one by one by the host, 6.2 at least, without a void
+// limit. A plane of a block of steps: 1.45 (measured 1.1 to 1.3), scalar rows 1.6 (1.5), of a remainder 1.2 and
+// 1.3 (1.0 and 1.25); the next block is 8.5 planes behind (7 to 10).
+// Laser-off epochs, chain and a launch per step: 200x200x192, 2 steps 475 and 272 us, 34 steps 816 and 594, 68 steps
+// 993 and 966, 170 steps 1778 and 2131, 680 steps 5289 and 8875; 1000x24x144, 10 steps 2296 and 281, 680 steps
+// 4904 and 5393; 48x48x144, 10 steps 190 and 110, 68 steps 287 and 335; 48x48x143, 34 steps 274 and 106, 680 steps
+// 2234 and 2340.
+static bool chain_pays(int nx, int ny, int nz, long long total, bool vec, bool whole, int nsm) {
+    const double vox = 1e-6 * nx * ny * nz;
+    const double step = whole ? std::max(6.2, vec ? 4.2 + 1.0 * vox : 4.0 + 3.1 * vox)
+                              : vec ? 4.2 + 0.7 * vox : 3.3 + 1.8 * vox;
+    const double plane = vec ? 1.45 : 1.6, tail = vec ? 1.2 : 1.3, lag = 8.5;
+    // units: one or more windows of z groups per 16 rows; blocks beyond those on the chip start as others end
+    const double units = (double)((ny + kChainRows - 1) / kChainRows) * std::max(1.0, nz / 240.0);
+    const double on_chip = std::max(1.0, std::floor(nsm / units));
+    const long long blocks = total / kChainHalo, rest = total % kChainHalo;
+    double chain = 10.0;
+    if (blocks > 0) {
+        const double march = nx + 2.0 * kChainHalo, turns = std::floor((blocks - 1) / on_chip);
+        chain += plane * (march + turns * std::max(march, lag * on_chip) + (blocks - 1 - turns * on_chip) * lag);
+    }
+    if (rest > 0) chain += tail * (nx + 2.0 * rest);
+    return chain < step * total;
+}
+
 int plume_policy_steps(const BdPlumeParams* p, int* n_steps, float* dt_step, float* decay_step) {
     const double idx2 = 1.0 / ((double)p->dx * p->dx), idy2 = 1.0 / ((double)p->dy * p->dy);
     const double idz2 = 1.0 / ((double)p->dz * p->dz);
@@ -1139,13 +1177,14 @@ int plume_launch(const BdPlumeParams* p, float* Ca, float* Cb, int n_substeps, c
         if (in_b) *in_b = (int)(total & 1);
         return BD_OK;
     }
-    if ((nz + 3) / 4 <= 255) {
+    const bool groups_in_byte = (nz + 3) / 4 <= 255;
+    int dev = 0, nsm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    const int slots = std::max(1, nsm);
+    if (groups_in_byte && chain_pays(nx, ny, nz, total, vec, full_first != 0, slots)) {
         const int n_yt = (ny + kChainRows - 1) / kChainRows;
         const ChainPlan plan = chain_plan(mask, nx, ny, nz);
-        int dev = 0, nsm = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        const int slots = std::max(1, nsm);
         k_plume_chain_bits<<<dim3(n_yt, nx), 256, 0, st>>>(mask, ny, nz, mz, zl, plan.bits);
         k_plume_chain_units<<<1, 1024, 0, st>>>(plan, nx, n_yt, (nz + 3) / 4);
         BD_CHECK_LAUNCH("k_plume_chain_units");
@@ -1167,11 +1206,16 @@ int plume_launch(const BdPlumeParams* p, float* Ca, float* Cb, int n_substeps, c
     const int xc = tune_value(BD_TUNE_PLUME_XC);
     const dim3 dgrid((nz + 31) / 32, (ny + PD_BY - 1) / PD_BY, (nx + xc - 1) / xc);
     const bool direct = vec && dgrid.y <= 65535;
+    const bool listed = direct && groups_in_byte;
+    uint8_t* zlist = mask + plume_zlist_offset(nx, ny, nz);
+    if (listed) k_plume_zlist<<<dim3(dgrid.y, dgrid.z), 256, 0, st>>>(mask, nx, ny, nz, mz, xc, zl, zlist);
     for (long long s = 0; s < total; ++s) {
         const float* in = (s & 1) ? Cb : Ca;
         float* out = (s & 1) ? Ca : Cb;
-        if (direct)
-            k_plume_direct<<<dgrid, 8 * PD_BY, 0, st>>>(in, out, mask, nx, ny, nz, mz, xc, tab, zl);
+        if (listed)
+            k_plume_direct<true><<<dgrid, 8 * PD_BY, 0, st>>>(in, out, mask, nx, ny, nz, mz, xc, tab, zl, zlist);
+        else if (direct)
+            k_plume_direct<false><<<dgrid, 8 * PD_BY, 0, st>>>(in, out, mask, nx, ny, nz, mz, xc, tab, zl, nullptr);
         else
             k_plume_step<<<dim3((ny + PM_TY - 1) / PM_TY, nx), dim3(PM_TZ, PM_TY), 0, st>>>(nx, ny, nz, mz, tab, in, out,
                                                                                             mask, zl);

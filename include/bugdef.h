@@ -377,16 +377,20 @@ BD_API int bd_engine_record(BdEngine* e, const BdRecordSpec* spec, void* slot, v
 #define BD_TUNE_MC_BLOCKS_PER_SM  0  /* persistent MC grid: 128-thread CTAs per SM, 1..16 (0 = occupancy
                                         limit); photons per thread = n_photons / (grid * 128)          */
 #define BD_TUNE_STENCIL_XC        1  /* most x-planes per CTA of the substep kernel, 1..64 (default 8)   */
-#define BD_TUNE_PLUME_XC          2  /* batched plume stage: x-planes per unit, 1..64 (default 4)       */
+#define BD_TUNE_PLUME_XC          2  /* batched plume stage, and BD_PLUME_KERNEL_DIRECT with a launch per
+                                        step: x-planes per unit, 1..64 (default 4)                     */
 #define BD_TUNE_PLUME_KERNEL      3  /* plume stage: BD_PLUME_KERNEL_DIRECT (default) or
                                         BD_PLUME_KERNEL_COMPACT (value 5 is not used)                   */
 #define BD_PLUME_KERNEL_DIRECT    4  /* one launch per stage: each CTA advances 16 rows by 4 FTCS steps in
-                                        one march along x, following the CTA with the steps before      */
+                                        one march along x, following the CTA with the steps before; a
+                                        launch per step where the stage has too few steps for that to be
+                                        shorter, or nz > 1020                                           */
 #define BD_PLUME_KERNEL_COMPACT   6  /* one launch per FTCS step: one wave of CTAs over a compact list of
                                         the live (column, band) units; once per stage the x planes per
                                         unit are chosen on the device (2..12, the smallest whose unit
                                         count fits one wave). Same results as BD_PLUME_KERNEL_DIRECT;
-                                        nz % 4 != 0 falls back to it                                    */
+                                        nz % 4 != 0, nz > 1020 or buffers that are not 16-byte aligned
+                                        fall back to it                                                 */
 #define BD_TUNE_STENCIL_CAP       4  /* at most this many substep CTAs per SM (0 = no cap, default): the
                                         plume stage runs beside the substeps and keeps the rest         */
 #define BD_TUNE_COUNT             5
