@@ -13,7 +13,7 @@
 //     photon by one event per loop iteration and takes a new photon as soon as its own ends, so
 //     warps stay full while the per-photon event counts differ by orders of magnitude;
 //   * a crossing is free of branches (the crossed axis by selection), interactions wait for company,
-//     and few photons are spread over all resident warps: a warp runs the union of its lanes' paths;
+//     and few photons are spread over half of the resident warps: a warp runs the union of its lanes' paths;
 //   * Philox-4x32-10 counter-based RNG keyed on (seed, photon index): no RNG state in memory
 //     and a photon's path does not depend on which thread traced it;
 //   * optical properties packed as one float4 {mu_t, mu_a/mu_t, g, n} per voxel read through
@@ -521,10 +521,15 @@ int mc_launch(const BdMcParams* p, const float* props, const uint8_t* flags, flo
         }
         const int want = tune_value(BD_TUNE_MC_BLOCKS_PER_SM);
         const int use_sm = want > 0 ? std::min(want, occ) : occ;
-        // a warp runs the union of its lanes' branches, so few photons finish sooner spread over all
-        // resident warps, a few lanes of each, than packed into full ones
-        blocks = std::max(1, std::min((int)std::min<long long>(p->n_photons, (long long)sm_count * use_sm), max_blocks));
-        const int lanes = (int)std::min<long long>(32, std::max<long long>(1, (p->n_photons + 4LL * blocks - 1) / (4LL * blocks)));
+        // A warp runs the union of its lanes' branches, so few photons finish sooner spread over half of the resident
+        // warps, some lanes of each, than packed into full ones; over all of them, photons whose histories are
+        // alike cost more issue slots than the union saves. 20 k / 40 k / 80 k photons over all, and over half:
+        // crater stack of 200x200x128 0.94 / 1.08 / 1.16 and 0.94 / 1.10 / 1.18 ms, one dense medium 0.63 / 0.68 /
+        // 0.74 and 0.55 / 0.56 / 0.59, a clear one 0.20 / 0.20 / 0.20 and 0.16 / 0.17 / 0.17 (full warps of the kernel
+        // before: 1.35 / 1.42 / 1.46, 0.67 / 0.71 / 0.84, 0.17 / 0.18 / 0.20).
+        const long long most = std::max(1LL, std::min<long long>((long long)sm_count * use_sm, max_blocks));
+        const int lanes = (int)std::min<long long>(32, std::max<long long>(1, (p->n_photons + 2 * most - 1) / (2 * most)));
+        blocks = (int)std::max(1LL, std::min(most, (p->n_photons + 4LL * lanes - 1) / (4LL * lanes)));
         BD_CUDA(cudaMemsetAsync(queue, 0, sizeof(unsigned long long), st));
         BD_CUDA(cudaMemsetAsync(partials, 0, sizeof(double) * BD_LEDGER_LEN * blocks, st));
         if (p->launch_axis == 0)
