@@ -177,17 +177,17 @@ def autotune(inst, epochs_per_trial: int = 6, candidates=None, device=None, log=
     MC CTAs per SM (photons per thread) are timed by whole laser-on epochs; x-planes per CTA of the
     fused substep kernel by whole epochs with the laser off (the void domain does not change between
     trials): the plume stage runs beside MC and the substeps, so a shape that slows its own stage
-    but leaves the plume more room can win. The plume kernel and BD_TUNE_PLUME_XC are searched
-    together, also by laser-off epochs; the compact kernel chooses its x-planes per stage on the
-    device. Sets
-    the winning values process-wide (bd_tune_set) and returns the choices with every trial's time
-    (ms per epoch)."""
+    but leaves the plume more room can win. The plume kernels are timed by laser-off epochs too, each as
+    often as the other. BD_TUNE_PLUME_XC is left as it is unless `candidates` names values for it
+    (then searched together with the direct kernel): a whole stage in one launch and the compact kernel
+    do not read it, only the batched stage and stages of few steps do. Sets the winning values
+    process-wide (bd_tune_set) and returns the choices with every trial's time (ms per epoch)."""
     from . import _lib
     cand = dict(candidates or {})
     cand.setdefault(_lib.TUNE_MC_BLOCKS_PER_SM, [1, 2, 3, 4, 6, 8])
     cand.setdefault(_lib.TUNE_STENCIL_XC, [1, 2, 4, 8, 16])
     cand.setdefault(_lib.TUNE_PLUME_KERNEL, [_lib.PLUME_KERNEL_DIRECT, _lib.PLUME_KERNEL_COMPACT])
-    cand.setdefault(_lib.TUNE_PLUME_XC, [2, 3, 4, 6])
+    cand.setdefault(_lib.TUNE_PLUME_XC, [None])
     cand.setdefault(_lib.TUNE_STENCIL_CAP, [0, 1, 2])
     names = {_lib.TUNE_MC_BLOCKS_PER_SM: "mc_ctas_per_sm", _lib.TUNE_STENCIL_XC: "stencil_xc",
              _lib.TUNE_PLUME_XC: "plume_xc", _lib.TUNE_PLUME_KERNEL: "plume_kernel",
@@ -219,9 +219,8 @@ def autotune(inst, epochs_per_trial: int = 6, candidates=None, device=None, log=
     # the MC trials, whose laser epochs deepen the crater, come last
     single(_lib.TUNE_STENCIL_XC, False)
     single(_lib.TUNE_STENCIL_CAP, False)
-    # plume kernel x x-planes per CTA (the knob shapes the batched stage only; the pair is searched so that a batched run is tuned too); the
-    # candidates differ by a few per cent, so each is timed twice (forward, then reversed order) and
-    # keeps its better time
+    # plume kernels; the candidates may differ by a few per cent, so each is timed twice (forward, then
+    # reversed order) and keeps its better time
     combos = [(int(kern), xc) for kern in cand[_lib.TUNE_PLUME_KERNEL]
               for xc in (cand[_lib.TUNE_PLUME_XC] if kern == _lib.PLUME_KERNEL_DIRECT else [None])]
     best_t = {}
