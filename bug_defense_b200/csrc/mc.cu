@@ -64,6 +64,8 @@ struct PhotonState {
 // The longest axis whose indices, and the one past its end, are exact in FP32: beyond it gx + 1 == gx, and
 // the photon's linear index would walk out of the grid unseen.
 constexpr int kMcMaxAxis = 1 << 24;
+// The largest event cap that a photon's 32-bit counter can reach.
+constexpr long long kMcMaxEvents = 0xffffffffLL;
 
 // Puts the exit face of an axis without motion out of reach: its distance is about 1e30 voxels.
 constexpr float kFar = 1e30f;
@@ -317,7 +319,7 @@ __global__ void __launch_bounds__(128, BD_MC_MIN_BLOCKS) k_mc_trace(McDev P, con
             else live = photon_launch<DEPTH>(P, (long long)p, props, latz, sl, s);
         }
         if (live && !hit) {
-            if (s.ev >= P.max_events) {
+            if (s.ev >= (unsigned)P.max_events) {   // at most kMcMaxEvents
                 // event cap reached: the remaining weight is accounted, not lost
                 atomicAdd(&sl[BD_LEDGER_TRUNCATED], (double)s.w);
                 live = false;
@@ -480,7 +482,7 @@ McDev mc_dev_params(const BdMcParams* p) {
     d.sigma = p->sigma_axis; d.radius = p->beam_radius; d.profile = p->beam_profile;
     d.n_amb = p->n_ambient; d.rmax2 = p->r_max_sq; d.options = p->options;
     d.n_photons = p->n_photons; d.offset = p->photon_offset;
-    d.max_events = (unsigned)std::min<long long>(p->max_events, 0xffffffffLL);
+    d.max_events = p->max_events;
     d.seed = p->seed;
     d.fnx = (float)p->nx; d.fny = (float)p->ny; d.fnz = (float)p->nz;
     Philox::keys((uint32_t)p->seed, (uint32_t)(p->seed >> 32), d.keys);
@@ -498,9 +500,10 @@ int mc_launch(const BdMcParams* p, const float* props, const uint8_t* flags, flo
     McDev d = mc_dev_params(p);
     const float4* pr = reinterpret_cast<const float4*>(props);
     int blocks = 1;
-    // k_mc_trace tests the bounds on voxel indices in FP32, exact up to 2^24; mc_fluence.cu's are integers
-    const bool long_axis = std::max(p->nx, std::max(p->ny, p->nz)) > kMcMaxAxis;
-    if (((d.options & BD_MC_TALLY_FLUENCE) != 0 && L != nullptr) || tally64 == nullptr || long_axis) {
+    // k_mc_trace tests the bounds on voxel indices in FP32, exact up to 2^24, and counts events in 32 bits;
+    // mc_fluence.cu's indices are integers and its events 64 bits
+    const bool wide = std::max(p->nx, std::max(p->ny, p->nz)) > kMcMaxAxis || p->max_events > kMcMaxEvents;
+    if (((d.options & BD_MC_TALLY_FLUENCE) != 0 && L != nullptr) || tally64 == nullptr || wide) {
         // FP32 sums in memory depend on the order of the deposits: these launches keep the event order of
         // mc_fluence.cu (its comment has both sides)
         if (int rc = mc_fluence_launch(d, pr, flags, A, tally64, L, latz, queue, partials, max_blocks, sm_count, st,

@@ -15,7 +15,7 @@ struct McDev {
     float n_amb, rmax2;
     int options;
     long long n_photons, offset;
-    unsigned max_events;
+    long long max_events;
     float fnx, fny, fnz;
     uint32_t keys[20];   // the seed's Philox round keys
     unsigned long long seed;

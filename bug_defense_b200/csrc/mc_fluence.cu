@@ -1,6 +1,6 @@
 // Photon tracer of the launches whose results are FP32 sums in memory: the track length (fluence), and the
-// absorbed map where no exact tally is kept; and of grids with an axis of more than 2^24 voxels, whose
-// indices mc.cu's FP32 cannot hold.
+// absorbed map where no exact tally is kept; and of grids with an axis of more than 2^24 voxels or event caps of
+// more than 32 bits, which mc.cu's indices and counter cannot hold.
 //
 // An FP32 sum of thousands of deposits depends on their order by up to 3e-6 of the map (2-norm, 75 k photons on
 // a 26x40x50 grid): the beam's voxels first take the photons' equal first chords. Two traces with this order
@@ -57,7 +57,7 @@ struct FluencePhoton {
     float x, y, z, ux, uy, uz, iux, iuy, iuz, tau, w;
     float4 pr;
     int ix, iy, iz, idx;
-    unsigned ev;
+    long long ev;
 };
 
 // Launch: transverse offsets, footprint test, entrance Fresnel split and refraction, first

@@ -1,0 +1,33 @@
+"""A photon's event cap of more than 32 bits: the launch runs the tracer with the 64-bit counter (a cap cut to 32
+bits would end a photon early that a caller allowed to go on), and gives the map of a cap that 32 bits hold."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("cap,kernel", [(2 ** 32 - 1, "k_mc_trace"), (2 ** 32, "k_mc_fluence"),
+                                        (2 ** 62, "k_mc_fluence")])
+def test_event_caps_keep_their_bits(gpu, cap, kernel):
+    import torch
+    from bug_defense_b200 import voxel_mc
+    from torch.profiler import ProfilerActivity, profile
+    shape = (18, 20, 24)
+    full = lambda v: np.full(shape, v)
+    props = voxel_mc.pack_props(full(2.0), full(15.0), full(0.85), full(1.4), torch.device("cuda"))
+
+    def run(max_events):
+        A = torch.zeros(int(np.prod(shape)), device="cuda")
+        p = voxel_mc.make_params(Nx=shape[0], Ny=shape[1], Nz=shape[2], Lx=0.5, Ly=0.5, Lz=0.6, n_photons=3000,
+                                 spot_dia=0.2, theta_inc_deg=15.0, seed=5, tally_fluence=False, max_events=max_events)
+        voxel_mc.trace(p, props, A)
+        torch.cuda.synchronize()
+        return A
+
+    want = run(10_000_000)
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        got = run(cap)
+    keys = [e.key for e in prof.key_averages()]
+    ran = {n for n in ("k_mc_trace", "k_mc_fluence") if any(f"{n}<" in key for key in keys)}
+    assert ran == {kernel}, keys
+    assert torch.equal(got, want) and float(got.sum()) > 0
