@@ -41,32 +41,62 @@ static std::atomic<int> g_tune_gen{0};
 int tune_value(int knob) { return g_tune[knob].load(std::memory_order_relaxed); }
 int tune_generation() { return g_tune_gen.load(std::memory_order_relaxed); }
 
-// The current device's scratch pool, created on first use; nullptr when it cannot be.
-static cudaMemPool_t scratch_pool() {
-    constexpr int kMaxDevices = 64;
-    static std::mutex mu;
-    static cudaMemPool_t pools[kMaxDevices] = {};
-    static bool tried[kMaxDevices] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
-    std::lock_guard<std::mutex> lock(mu);
-    if (!tried[dev]) {
-        tried[dev] = true;
-        cudaMemPoolProps props = {};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = dev;
-        cudaMemPool_t pool = nullptr;
-        cuuint64_t keep = kScratchKeep;
-        if (cudaMemPoolCreate(&pool, &props) == cudaSuccess) {
-            if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess)
-                pools[dev] = pool;
-            else
-                cudaMemPoolDestroy(pool);
-        }
-        if (!pools[dev]) cudaGetLastError();
+// The current context's id, another after every cudaDeviceReset; 0 when it cannot be had.
+static unsigned long long context_id() {
+    typedef CUresult (*GetIdFn)(CUcontext, unsigned long long*);
+    static const GetIdFn get_id = []() -> GetIdFn {
+        // looked up through the runtime: the library does not link libcuda, and loads without a driver
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        const bool ok = cudaGetDriverEntryPoint("cuCtxGetId", &fn, cudaEnableDefault, &found) == cudaSuccess &&
+                        found == cudaDriverEntryPointSuccess;
+        if (!ok) cudaGetLastError();
+        return ok ? reinterpret_cast<GetIdFn>(fn) : nullptr;
+    }();
+    unsigned long long id = 0;
+    if (!get_id) return 0;
+    if (get_id(nullptr, &id) == CUDA_SUCCESS) return id;
+    // no context yet, or a reset took it: the runtime makes one
+    if (cudaFree(nullptr) != cudaSuccess || get_id(nullptr, &id) != CUDA_SUCCESS) {
+        cudaGetLastError();
+        return 0;
     }
-    return pools[dev];
+    return id;
+}
+
+// The current context's scratch pool, created on first use; nullptr when it cannot be. A pool does not outlive
+// its context, so a reset device gets another; past kMaxContexts of them calls do without.
+static cudaMemPool_t scratch_pool() {
+    constexpr int kMaxContexts = 256;
+    static std::mutex mu;
+    static struct {
+        unsigned long long id;
+        cudaMemPool_t pool;
+    } pools[kMaxContexts] = {};
+    static int n_pools = 0;
+    const unsigned long long id = context_id();
+    int dev = 0;
+    if (id == 0 || cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+    std::lock_guard<std::mutex> lock(mu);
+    for (int i = 0; i < n_pools; ++i)
+        if (pools[i].id == id) return pools[i].pool;
+    if (n_pools == kMaxContexts) return nullptr;
+    auto& slot = pools[n_pools++];
+    slot.id = id;
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    cuuint64_t keep = kScratchKeep;
+    if (cudaMemPoolCreate(&pool, &props) == cudaSuccess) {
+        if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess)
+            slot.pool = pool;
+        else
+            cudaMemPoolDestroy(pool);
+    }
+    if (!slot.pool) cudaGetLastError();
+    return slot.pool;
 }
 
 cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t st) {

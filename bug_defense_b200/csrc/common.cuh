@@ -74,12 +74,12 @@ inline size_t plume_mask_bytes(int nx, int ny, int nz) {
     return plume_chain_offset(nx, ny, nz) + plume_chain_bytes(nx, ny, nz);
 }
 
-// Stream-ordered scratch of the synchronous entry points (error flags, the plume's masks and lists),
-// from one pool per device that keeps up to kScratchKeep bytes mapped between calls; what a call
-// needs beyond that goes back to the driver at the next synchronisation. The default pool keeps
-// nothing: every one of these calls ends in a synchronisation, so each call mapped and unmapped its
-// few bytes again (thermal 64x64x128, 20 substeps: 750-1520 us a call for 295 us of kernels; see
-// scratch_alloc). Safe from any thread and stream: the pool orders reuse by stream.
+// Stream-ordered scratch of the synchronous entry points (the plume's masks and plans, the convolutions' error
+// flags), from one pool per context that keeps up to kScratchKeep bytes mapped between calls; what a call needs
+// beyond that goes back to the driver at the next synchronisation. The default pool keeps nothing: every one of
+// these calls ends in a synchronisation, so each call mapped and unmapped its few bytes again (a convolution of
+// an 8x8x8 volume 450 us a call, 40 us so; one plume step of a 24x24x32 grid 525 and 60). Safe from any thread and
+// stream: the pool orders reuse by stream.
 constexpr unsigned long long kScratchKeep = 32ull << 20;
 cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t st);
 
