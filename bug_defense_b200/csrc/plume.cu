@@ -12,6 +12,7 @@
 //   k_plume_direct_c  (BD_PLUME_KERNEL_COMPACT): one launch per step, one wave of CTAs looping over a
 //                     compact list of the live units, x planes per unit chosen per stage
 // Layout: C-order (nx, ny, nz), z fastest; the neighbourhood of every voxel is one mask byte.
+#include "chain_wait.cuh"
 #include "common.cuh"
 #include "engine.cuh"
 
@@ -591,7 +592,6 @@ constexpr int kChainR = 2;                                     // rows of a warp
 constexpr int kChainWarps = (kChainRows + 2 * kChainHalo) / kChainR;
 constexpr int kChainThreads = 32 * kChainWarps;
 constexpr int chain_smem_bytes(int S) { return 2 * S * 2 * kChainWarps * 32 * (int)sizeof(float4); }
-constexpr unsigned kChainPolls = 1u << 22;                     // polls of ~0.7 us: about 3 s, then an error
 constexpr int kChainDone = 0x7fffffff;
 
 struct ChainUnit {
@@ -625,26 +625,6 @@ static ChainPlan chain_plan(uint8_t* mask, int nx, int ny, int nz) {
     p.progress = reinterpret_cast<int*>(at);
     p.cap = (int)plume_chain_capacity(ny, nz);
     return p;
-}
-
-__device__ __forceinline__ int ld_acquire(const int* p) {
-    int v;
-    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_release(int* p, int v) {
-    asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-// Waits until *p > plane; false when the polls run out or another wait already has.
-__device__ __forceinline__ bool chain_wait(const int* p, int plane, int& seen, int* err) {
-    for (unsigned it = 0; it < kChainPolls; ++it) {
-        seen = ld_acquire(p);
-        if (seen > plane) return true;
-        if ((it & 255u) == 255u && ld_acquire(err) != 0) return false;
-    }
-    atomicExch(err, 1);
-    return false;
 }
 
 // The field is written by other SMs during the kernel: it is read past the L1.

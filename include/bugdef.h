@@ -402,6 +402,9 @@ BD_API int bd_tune_get(int knob, int* value);
  * nothing arrives on (arrive = 0: returns BD_ERR_TIMEOUT) or that it completed itself (arrive = 1:
  * BD_OK). Synchronises `stream`; the context stays usable after the timeout. */
 BD_API int bd_selftest_wait_timeout(int max_polls, int arrive, void* stream);
+/* The same for the chained plume kernel's wait on progress in global memory: a warp waits for 32 progress
+ * words that nobody advances (arrive = 0) or that one of its lanes does (arrive = 1). */
+BD_API int bd_selftest_chain_wait_timeout(int max_polls, int arrive, void* stream);
 
 /* ---------------------------------------------------------------------------------------------
  * Absorbed-map denoiser: 3-D convolution layers (tcgen05 BF16 tensor cores, FP32 accumulation).
