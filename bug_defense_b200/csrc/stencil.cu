@@ -388,6 +388,9 @@ static void launch_substeps(const Geo& g, const AblConst& c, float* Ta, float* T
     else run(std::false_type{});
 }
 
+// The scale of the heat source; without one the kernel scales zeros, which an infinite or NaN scale must not reach.
+static float source_scale(int is_active, float q_scale) { return is_active ? q_scale : 0.0f; }
+
 // The synchronous entry points' end: waits for the launches and reports what went wrong in them.
 static int finish(int rc, cudaStream_t st, const char* what) {
     if (rc) return rc;
@@ -411,7 +414,7 @@ extern "C" int bd_thermal_advance(const BdThermalParams* p, float* Ta, float* Tb
     if (n == 0) return BD_OK;
     Geo g = make_geo(p->nx, p->ny, p->nz, p->dx, p->dy, p->dz, p->dt, p->h_eff, p->t_ambient);
     AblConst c{};
-    c.q_scale = p->q_scale;
+    c.q_scale = source_scale(p->is_active, p->q_scale);
     c.is_active = p->is_active;
     cudaStream_t st = as_stream(stream);
     if (p->bc_mode == BD_BC_SERIES)
@@ -436,7 +439,7 @@ int ablation_launch(const BdAblationParams* p, float* Ta, float* Tb, int n, floa
                     const uint8_t* F, const float* src, const float* K, const float* R, cudaStream_t st) {
     Geo g = make_geo(p->nx, p->ny, p->nz, p->dx, p->dy, p->dz, p->dt, p->h_eff, p->t_ambient);
     AblConst c;
-    c.t_abl = p->t_abl; c.t_void = p->t_void; c.q_scale = p->q_scale;
+    c.t_abl = p->t_abl; c.t_void = p->t_void; c.q_scale = source_scale(p->is_active, p->q_scale);
     c.arr_A = p->arr_A; c.arr_EaR = p->arr_Ea_over_R; c.char_A = p->char_A; c.char_EaR = p->char_Ea_over_R;
     c.zero_src_in_ablated = p->zero_src_in_ablated; c.is_active = p->is_active;
     c.t_cold = p->has_char ? char_cold_limit(p->char_A, p->char_Ea_over_R, p->dt) : 0.0f;
