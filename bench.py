@@ -237,6 +237,25 @@ def algorithmic_bytes(eng, n_void):
     return {"substep": sub, "plume_step": plume}
 
 
+def mc_alone_ms(eng, n=4):
+    """Device time of the MC stage (ms per laser epoch) with the plume stage after the substeps on the same stream,
+    and the photon-steps of such an epoch: in the timed run the stages share the chip, and MC's span is mostly
+    waiting for the plume's launch to leave its SMs."""
+    from bug_defense_b200 import _lib
+    lib = _lib.load()
+    keep, eng.serial_plume, eng.power = (eng.serial_plume, eng.power), True, POWER_W
+    eng._enqueue(0)
+    lib.bd_engine_timing(eng._handle, 1)
+    for _ in range(n):
+        eng._enqueue(0)
+    stage, nep = (ctypes.c_double * 4)(), ctypes.c_int64(0)
+    _lib.check(lib.bd_engine_timing_read(eng._handle, stage, ctypes.byref(nep)))
+    lib.bd_engine_timing(eng._handle, 0)
+    led = eng._diag(None)["ledger"]
+    eng.serial_plume, eng.power = keep
+    return stage[0] / max(int(nep.value), 1), float(led[_lib.LEDGER_COLLISIONS] + led[_lib.LEDGER_CROSSINGS])
+
+
 def run_ours(args, rank, world, local):
     import torch
     import torch.distributed as dist
@@ -403,13 +422,16 @@ def ours_main(args):
     bytes_per_launch = ab["substep"] if dom == "substeps" else ab["plume_step"]
     achieved = bytes_per_launch / (per_launch[dom] * 1e-3) / 1e9
     from bug_defense_b200 import _lib
+    # warp instructions the chip can issue per second: SMs x 4 schedulers x clock
+    mhz = (r["clocks"] or {}).get("sm_mhz") or 1965.0
+    issue_peak = torch.cuda.get_device_properties(eng.dev).multi_processor_count * 4 * mhz * 1e6
     kv = ctypes.c_int(0)
     _lib.call("bd_tune_get", _lib.TUNE_PLUME_KERNEL, ctypes.byref(kv))
     plume_kernel = {4: "k_plume_chain", 6: "k_plume_direct_c"}.get(kv.value, "k_plume_step")
     traffic = None
     tf = ROOT / "profiles" / "traffic.json"
-    if tf.exists():
-        tj = json.loads(tf.read_text())
+    tj = json.loads(tf.read_text()) if tf.exists() else {}
+    if tj:
         key = {"substeps": "k_substep", "plume": plume_kernel.split("<")[0]}[dom]
         if key in tj:
             traffic = tj[key]["bytes_per_voxel"] * eng.Nx * eng.Ny * eng.Nz
@@ -420,38 +442,40 @@ def ours_main(args):
             "avg_launch_ms": round(per_launch[dom], 5),
             "units_per_launch": ("voxel-substeps" if dom == "substeps" else "plume (void) voxel-steps"),
             "void_voxels": int(n_void)}
-    if dom == "plume":
-        if plume_kernel == "k_plume_chain":
-            roof["launch"] = "one launch runs the stage; bytes and ms are a step's"
+    chain_wipv = tj.get("k_plume_chain", {}).get("warp_instructions_per_voxel_step")
+    if dom == "plume" and plume_kernel == "k_plume_chain":
+        # one launch runs the stage and keeps its planes on chip for four steps: DRAM and L2 do not bound it
+        # (0.3 and 12 % in ncu), the issue of dependent operations does
+        ips = chain_wipv * n_void / (per_launch[dom] * 1e-3) if chain_wipv else None
+        roof.update({"bound": "issue", "achieved": ips and round(ips / 1e9, 1), "peak": round(issue_peak / 1e9, 1),
+                     "unit": "G warp instructions/s", "frac": ips and round(ips / issue_peak, 4),
+                     "peak_source": "SMs x 4 schedulers x SM clock; instructions per voxel-step from one ncu capture "
+                                    "(profiles/traffic.json)",
+                     "launch": "one launch runs the stage; instructions, bytes and ms are a step's"})
+    elif dom == "plume":
         l2 = l2_copy_gbs(eng.dev)
         roof.update({"l2_peak": round(l2, 1), "l2_frac": round(achieved / l2, 4),
                      "l2_method": "best of 8, 16 and 32 MB device-to-device copies (L2-resident pairs), 100 "
                                   "copies replayed from one CUDA graph, read + written bytes / event time, "
                                   "measured in this run"})
     led = r["last_diag"]["ledger"]
-    mc_ms = stage[0]
-    photons = r["n_on"] * eng.n_photons
-    mc = {"photons_per_s": photons / (mc_ms * 1e-3) if mc_ms > 0 else None,
-          "mc_ms_per_laser_epoch": mc_ms / max(r["n_on"], 1)}
+    mc_ms, steps_per_epoch = mc_alone_ms(eng)
+    mc = {"photons_per_s": eng.n_photons / (mc_ms * 1e-3) if mc_ms > 0 else None,
+          "mc_ms_per_laser_epoch": round(mc_ms, 4),
+          "mc_ms_note": "the MC stage with the plume stage after it, measured behind the timed region",
+          "mc_span_ms_per_timed_laser_epoch": round(stage[0] / max(r["n_on"], 1), 4)}
     if r["laser_diag"] is not None:
-        from bug_defense_b200 import _lib as L_
         ld = r["laser_diag"]["ledger"]
-        steps_per_epoch = float(ld[L_.LEDGER_COLLISIONS] + ld[L_.LEDGER_CROSSINGS])
         mc["photon_steps_per_laser_epoch"] = steps_per_epoch
         if mc_ms > 0:
-            mc["photon_steps_per_s"] = steps_per_epoch * r["n_on"] / (mc_ms * 1e-3)
+            mc["photon_steps_per_s"] = steps_per_epoch / (mc_ms * 1e-3)
         lc = (ld[1:7].sum() + ld[8] + ld[9] - ld[7]) / max(ld[0], 1)
         mc["ledger_closure_minus_1"] = float(lc - 1.0)
-        # issue-rate roof: SMs x 4 schedulers x 1 warp instruction per clock x 32 lanes / thread
-        # instructions per photon-step (the count of one ncu capture, profiles/traffic.json)
-        tf = ROOT / "profiles" / "traffic.json"
-        ipp = json.loads(tf.read_text()).get("k_mc_trace", {}).get("thread_instructions_per_photon_step") \
-            if tf.exists() else None
+        # issue-rate roof: warp instructions the chip can issue x 32 lanes / thread instructions per
+        # photon-step (the count of one ncu capture, profiles/traffic.json)
+        ipp = tj.get("k_mc_trace", {}).get("thread_instructions_per_photon_step")
         if ipp and mc_ms > 0:
-            import torch
-            n_sm = torch.cuda.get_device_properties(eng.dev).multi_processor_count
-            mhz = (r["clocks"] or {}).get("sm_mhz") or 1965.0
-            roof_steps = n_sm * 4 * mhz * 1e6 * 32 / ipp
+            roof_steps = issue_peak * 32 / ipp
             mc["issue_roof_photon_steps_per_s"] = roof_steps
             mc["issue_roof_frac"] = round(mc["photon_steps_per_s"] / roof_steps, 4)
             mc["thread_instructions_per_photon_step"] = ipp
@@ -538,9 +562,8 @@ def denoised_run_leg(n_laser=10, check_every=5):
         row["speedup"] = round(row["plain_ms_per_laser_epoch"] / row["denoised_ms_per_laser_epoch"], 3)
         out.append(row)
     return {"runs": out, "laser_epochs_timed": n_laser,
-            "note": "laser-on epochs of the full-resolution coupled run; the plume stage (one launch for all "
-                    "its FTCS steps, beside MC and the substeps) bounds the epoch, so a cheaper optical step shortens "
-                    "the epoch only by what it removes from the plume stream's competition"}
+            "note": "laser-on epochs of the full-resolution coupled run; the plume stage is one launch that keeps every "
+                    "SM until it ends, so the optical step and the substeps mostly follow it and their times add up"}
 
 
 def campaign_main(args):
