@@ -176,8 +176,8 @@ def autotune(inst, epochs_per_trial: int = 6, candidates=None, device=None, log=
     campaign instance dict or a callable returning an engine with a `laser_power` attribute.
     MC CTAs per SM (photons per thread) are timed by whole laser-on epochs; x-planes per CTA of the
     fused substep kernel by whole epochs with the laser off (the void domain does not change between
-    trials): the plume stage runs beside MC and the substeps, so a shape that slows its own stage
-    but leaves the plume more room can win. The plume kernels are timed by laser-off epochs too, each as
+    trials): a plume stage of a launch per step runs beside MC and the substeps, so a shape that slows
+    its own stage but leaves the plume more room can win. The plume kernels are timed by laser-off epochs too, each as
     often as the other. BD_TUNE_PLUME_XC is left as it is unless `candidates` names values for it
     (then searched together with the direct kernel): a whole stage in one launch and the compact kernel
     do not read it, only the batched stage and stages of few steps do. Sets the winning values

@@ -853,7 +853,7 @@ int conv_check(const BdConvCall& c) {
     BD_REQUIRE(c.nx > 0 && c.ny > 0 && c.nz > 0, "bd_conv3d: dims must be positive");
     BD_REQUIRE(c.cin == 16 || c.cin == 32 || c.cin == 64, "bd_conv3d: cin must be 16, 32 or 64");
     BD_REQUIRE(c.n_slice == 16 || c.n_slice == 32 || c.n_slice == 64, "bd_conv3d: n_slice must be 16, 32 or 64");
-    BD_REQUIRE(!(c.cin == 64 && c.n_slice == 64), "bd_conv3d: cin 64 x n_slice 64 exceeds shared memory; split the slice");
+    BD_REQUIRE(!(c.cin == 64 && c.n_slice == 64), "bd_conv3d: cin 64 x n_slice 64 is not supported; split the slice");
     BD_REQUIRE(c.n_off >= 0 && c.n_off + c.n_slice <= c.cout_total && c.n_off % 8 == 0, "bd_conv3d: bad output slice");
     BD_REQUIRE(c.taps == 27 || c.taps == 9, "bd_conv3d: taps must be 27 or 9");
     BD_REQUIRE(c.mode >= BD_CONV_FWD_RELU && c.mode <= BD_CONV_BWD_UPADD, "bd_conv3d: unknown mode");

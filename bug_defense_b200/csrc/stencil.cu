@@ -14,8 +14,8 @@
 // warps. A face's flux is computed once: +x kept for the next plane, z faces within the thread and
 // by shuffle from the lane below, only the y faces twice (their rows come from L1). The source and the
 // enthalpy are read only where a voxel uses them.
-// What bounds it: latency and issue, with DRAM behind them (200x200x192: 217 MB a substep, 4 TB/s;
-// 575 warp instructions per 32 groups of 4). 20 substeps, char on / char and damage on: 1.85 / 2.13 ms
+// What bounds it: latency and issue, with DRAM behind them (200x200x192: 172 MB of DRAM a substep, 3.1 TB/s;
+// 527 warp instructions per 32 groups of 4, issue 57 %). 20 substeps, char on / char and damage on: 1.85 / 2.13 ms
 // by 32 x 16 tiles staged through shared memory with every face computed twice, now 1.07 / 1.33 ms
 // (5 CTAs of 128 threads per SM; 3 of 256 1.20 / 1.51, 6 of 128 1.17 / 1.46, 10 of 64 1.09 / 1.34).
 // 150x150x138 (rows of no whole float4s) 0.86 -> 0.64 ms. Same bits.
@@ -35,8 +35,9 @@ struct Geo {
 
 // Harmonic face conductance 2 k_c k_n / (k_c + k_n + 1e-12) by the approximate reciprocal (<= 1 ulp): six
 // precise IEEE divisions per voxel made the stencil instruction-bound, while the parity bar on T is
-// 1e-4 relative. The operations are written out: the compiler contracts none of them, so every
-// grid and every launch shape gives the same bits.
+// 1e-4 relative. The operations are written out: the compiler contracts none of them, so the launch
+// shape does not change a bit. The load width does, by a rounding of the -y face in half of the rows (see
+// `fuse`): a grid of whole float4 rows rounds otherwise where its buffers are not aligned.
 __device__ __forceinline__ float rcp_approx(float x) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -337,9 +338,11 @@ static Geo make_geo(int nx, int ny, int nz, float dx, float dy, float dz, float 
     return g;
 }
 
-// Unused dynamic shared memory that lets at most `cap` substep CTAs share an SM (0: no cap). The
-// plume stage runs beside the substeps; capping them leaves the plume's CTAs room on every SM (16 KB
-// of shared memory per SM stay free for them). The kernel's limit is raised once per instantiation.
+// Unused dynamic shared memory that lets at most `cap` substep CTAs share an SM (0: no cap). A plume stage
+// of a launch per step runs beside the substeps, and capping them leaves its CTAs room on every SM (16 KB of
+// shared memory per SM stay free for them). The chained plume kernel shares an SM with no substep CTA (it
+// takes the registers), so beside it a cap only slows the substeps: laser-off epochs of 200x200x192 6.3 and
+// 8.0 ms with 2 and 1 CTAs per SM, 5.3 without. The kernel's limit is raised once per instantiation.
 static size_t substep_pad_bytes(int cap, const void* kernel) {
     if (cap <= 0) return 0;
     int dev = 0, per_sm = 0, per_block = 0;

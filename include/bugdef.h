@@ -375,8 +375,9 @@ BD_API int bd_engine_record(BdEngine* e, const BdRecordSpec* spec, void* slot, v
  * every launch; results do not depend on them beyond the order of FP32 atomic tally additions. A
  * change bumps a generation counter so engines re-capture their epoch graphs. */
 #define BD_TUNE_MC_BLOCKS_PER_SM  0  /* persistent MC grid: 128-thread CTAs per SM, 1..16 (0 = occupancy
-                                        limit); photons per thread = n_photons / (grid * 128)          */
-#define BD_TUNE_STENCIL_XC        1  /* most x-planes per CTA of the substep kernel, 1..64 (default 8)   */
+                                        limit); few photons take fewer CTAs, some lanes of each warp   */
+#define BD_TUNE_STENCIL_XC        1  /* most x-planes per CTA of the substep kernel, 1..64 (default 8);
+                                        grids that would leave the chip idle take fewer                 */
 #define BD_TUNE_PLUME_XC          2  /* batched plume stage, and BD_PLUME_KERNEL_DIRECT with a launch per
                                         step: x-planes per unit, 1..64 (default 4)                     */
 #define BD_TUNE_PLUME_KERNEL      3  /* plume stage: BD_PLUME_KERNEL_DIRECT (default) or
@@ -391,8 +392,9 @@ BD_API int bd_engine_record(BdEngine* e, const BdRecordSpec* spec, void* slot, v
                                         count fits one wave). Same results as BD_PLUME_KERNEL_DIRECT;
                                         nz % 4 != 0, nz > 1020 or buffers that are not 16-byte aligned
                                         fall back to it                                                 */
-#define BD_TUNE_STENCIL_CAP       4  /* at most this many substep CTAs per SM (0 = no cap, default): the
-                                        plume stage runs beside the substeps and keeps the rest         */
+#define BD_TUNE_STENCIL_CAP       4  /* at most this many substep CTAs per SM (0 = no cap, default): a plume
+                                        stage of a launch per step runs beside the substeps and keeps the
+                                        rest; a stage in one launch shares an SM with none              */
 #define BD_TUNE_COUNT             5
 BD_API int bd_tune_set(int knob, int value);
 BD_API int bd_tune_get(int knob, int* value);
